@@ -645,7 +645,7 @@ klft_status klft_run_metropolis(klft_lattice *lat, double beta, double delta, in
   WilsonPlan tplan;
   size_t toff = 0;
   if (ntw > 0) {
-    klft_status s = make_wilson_plan(lat, temporal_pairs, ntemporal, nd - 1, tplan, toff);
+    klft_status s = make_wilson_plan(lat, temporal_pairs, ntemporal, nd - 1, tplan, toff, nd - 1);
     if (s != KLFT_OK) return s;
     toff += 2 * (size_t)ntemporal;
   }

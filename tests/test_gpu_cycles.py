@@ -82,3 +82,26 @@ def test_run_metropolis_fused_matches_single_calls(L, nc, precision, planar):
     np.testing.assert_array_equal(a.download(), b.download())
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("L,nc", [([16, 16, 16, 8], 3), ([12, 10, 8, 20], 2)])
+def test_run_metropolis_temporal_loops_have_room_for_every_plane(L, nc):
+    """The temporal loops of a run write one U' field and one set of partial sums
+    per spatial plane; at these sizes a single plane's scratch is smaller than
+    what the three planes write.  A lattice created beside it stays as it was."""
+    prop = "exp" if nc == 3 else "reference"
+    tp = [(l, t) for l in range(1, 5) for t in range(1, 5)]
+    a = GaugeField(L, nc, "fp64", "hot", 91)
+    b = GaugeField(L, nc, "fp64", "hot", 91)
+    for g in (a, b):
+        g.set_stream(91, 0)
+    c = GaugeField(L, nc, "fp64", "hot", 92)
+    before = c.download()
+    acc, plaq, wt, _, _ = a.run_metropolis_measured(5.0, 0.2, 2, 4, 1, prop, 0.25, True, tp)
+    for step in range(4):
+        assert acc[step] == b.metropolis(5.0, 0.2, 2, 1, prop, 0.25)[0]
+        if step:
+            assert plaq[step - 1] == b.plaquette()
+            np.testing.assert_array_equal(wt[step - 1], b.wilson_loop_temporal(tp))
+    np.testing.assert_array_equal(a.download(), b.download())
+    np.testing.assert_array_equal(c.download(), before)
