@@ -49,6 +49,13 @@ enum StreamKind : uint32_t {
   KIND_SWAP = 5u,        // per (cycle, pair): replica swap uniform
 };
 
+// 53-bit uniform in [0,1) from two words of a Philox block.
+KLFT_HD double u53(uint32_t hi, uint32_t lo) {
+  return (double)((((uint64_t)hi << 32) | lo) >> 11) * 0x1.0p-53;
+}
+// Kokkos drand(start, end) = start + (end - start) * u
+KLFT_HD double drand_u(double a, double b, double u) { return a + (b - a) * u; }
+
 // Sequential stream of 53-bit uniforms in [0,1).  key = (lo32(seed),
 // hi32(seed) ^ lo32(chain)), counter = (block, site, step, kind<<24 | sub).
 // Each Philox block gives two doubles, (w0:w1) then (w2:w3).
@@ -59,6 +66,13 @@ struct Stream {
   KLFT_HD Stream(uint64_t seed, uint64_t chain, uint32_t site_, uint32_t step_, uint32_t kind, uint32_t sub)
       : k0((uint32_t)seed), k1((uint32_t)(seed >> 32) ^ (uint32_t)chain), site(site_), step(step_),
         tag((kind << 24) | (sub & 0xFFFFFFu)), block(0), avail(0) {}
+  // number of the next uniform, and a jump to uniform p
+  KLFT_HD uint32_t position() const { return 2u * block - (uint32_t)avail; }
+  KLFT_HD void seek(uint32_t p) {
+    block = p >> 1;
+    avail = 0;
+    if (p & 1) (void)next();
+  }
   KLFT_HD double next() {
     if (avail == 0) {
       w[0] = block; w[1] = site; w[2] = step; w[3] = tag;
@@ -69,10 +83,9 @@ struct Stream {
     const uint32_t hi = avail == 2 ? w[0] : w[2];
     const uint32_t lo = avail == 2 ? w[1] : w[3];
     --avail;
-    return (double)((((uint64_t)hi << 32) | lo) >> 11) * 0x1.0p-53;
+    return u53(hi, lo);
   }
-  // Kokkos drand(start, end) = start + (end - start) * u
-  KLFT_HD double drand(double a, double b) { return a + (b - a) * next(); }
+  KLFT_HD double drand(double a, double b) { return drand_u(a, b, next()); }
   // Box-Muller pair
   KLFT_D void gauss2(double &g0, double &g1) {
     const double u0 = next(), u1 = next();
@@ -81,6 +94,23 @@ struct Stream {
     sincos(6.283185307179586 * u1, &s, &c);
     g0 = r * c;
     g1 = r * s;
+  }
+};
+
+// The same stream by position: uniform number p of a (kind, step, site) stream
+// (sub-stream 0) is half p & 1 of block p >> 1.
+struct SiteStream {
+  uint32_t k0, k1, site, step, tag;
+  KLFT_HD SiteStream(uint64_t seed, uint64_t chain, uint32_t site_, uint32_t step_, uint32_t kind)
+      : k0((uint32_t)seed), k1((uint32_t)(seed >> 32) ^ (uint32_t)chain), site(site_), step(step_), tag(kind << 24) {}
+  KLFT_HD Stream stream() const {
+    return Stream(((uint64_t)k1 << 32) | k0, 0, site, step, tag >> 24, 0);
+  }
+  KLFT_HD void block(uint32_t b, double &a, double &c) const {
+    uint32_t w[4] = {b, site, step, tag};
+    philox4x32_10(w, k0, k1);
+    a = u53(w[0], w[1]);
+    c = u53(w[2], w[3]);
   }
 };
 

@@ -13,18 +13,22 @@ constexpr double K2PI = 6.283185307179586;
 enum Proposal : int { PROPOSAL_REFERENCE = 0, PROPOSAL_EXP = 1 };
 
 // ------------------------------------------------------------------ proposals
+// The proposals read NPROP<NC> consecutive uniforms of the site's stream (SU(3):
+// 12 unless a drawn vector has norm zero); the accept uniform, when drawn, follows.
+template <int NC> struct RefDraws { static constexpr int n = NC == 1 ? 1 : (NC == 2 ? 3 : 12); };
+
 // U(1): exp(i phi), phi uniform in [-delta*pi, delta*pi]   (SUN.hpp:163-171)
-template <typename T> KLFT_D Mat<1, T> propose(Stream &g, const Mat<1, T> *, double delta, int, double) {
-  const double phi = g.drand(-delta * KPI, delta * KPI);
+template <typename T> KLFT_D Mat<1, T> propose(const double *u, double delta, const Mat<1, T> *) {
+  const double phi = drand_u(-delta * KPI, delta * KPI, u[0]);
   Mat<1, T> r;
   r.e[0][0] = mk<T>((T)cos(phi), (T)sin(phi));
   return r;
 }
 // SU(2): cos(a) + i sin(a) n.sigma  (SUN.hpp:174-189)
-template <typename T> KLFT_D Mat<2, T> propose(Stream &g, const Mat<2, T> *, double delta, int, double) {
-  const T alpha = (T)g.drand(0.0, delta * 2 * KPI);
-  const T u = (T)g.drand(-1.0, 1.0);
-  const T theta = (T)g.drand(0.0, 2.0 * KPI);
+template <typename T> KLFT_D Mat<2, T> propose(const double *w, double delta, const Mat<2, T> *) {
+  const T alpha = (T)drand_u(0.0, delta * 2 * KPI, w[0]);
+  const T u = (T)drand_u(-1.0, 1.0, w[1]);
+  const T theta = (T)drand_u(0.0, 2.0 * KPI, w[2]);
   const T salpha = sin(alpha);
   const T su = sqrt(T(1) - u * u);
   const T n1 = su * sin(theta);
@@ -32,57 +36,76 @@ template <typename T> KLFT_D Mat<2, T> propose(Stream &g, const Mat<2, T> *, dou
   Mat<2, T> r;
   r.e[0][0] = mk<T>(cos(alpha), u * salpha);
   r.e[0][1] = mk<T>(n1 * salpha, n2 * salpha);
-  r.e[1][0] = mk<T>(-r.e[0][1].re, r.e[0][1].im);
-  r.e[1][1] = mk<T>(r.e[0][0].re, -r.e[0][0].im);
+  su2_row1(r);
   return r;
 }
 // SU(3): reference Gram-Schmidt proposal (SUN.hpp:192-251); the exp(i eps H)
-// proposal has its own fixed-position stream (expprop.cuh).
-template <typename T> KLFT_D Mat<3, T> propose(Stream &g, const Mat<3, T> *, double delta, int, double) {
-  Mat<3, T> r;
-  T r1[6], r2[6], norm, fact;
-  cx<T> z1[3], z2[3], z3[3], z;
-  // The rejection loops of the reference end once a draw has nonzero norm; they
-  // are bounded here (the host rejects delta <= 0, for which they never end).
-  for (int tries = 0; tries < 64; ++tries) {
+// proposal has its own fixed-position stream (expprop.cuh).  The reference draws
+// a vector again while its norm is zero.  next() gives the uniforms in order;
+// false: a first draw had norm zero (the caller then redraws in stream order).
+template <typename T, typename Next> KLFT_D bool su3_vec(Next &next, double delta, T v[6], T &norm) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) r1[i] = (T)g.drand(0.0, delta);
-    norm = sqrt(r1[0] * r1[0] + r1[1] * r1[1] + r1[2] * r1[2] + r1[3] * r1[3] + r1[4] * r1[4] + r1[5] * r1[5]);
-    if (T(1) != (T(1) + norm)) break;
-  }
-  fact = T(1) / norm;
-  z1[0] = fact * mk<T>(r1[0], r1[1]);
-  z1[1] = fact * mk<T>(r1[2], r1[3]);
-  z1[2] = fact * mk<T>(r1[4], r1[5]);
-  for (int outer = 0; outer < 64; ++outer) {
-    for (int tries = 0; tries < 64; ++tries) {
-#pragma unroll
-      for (int i = 0; i < 6; ++i) r2[i] = (T)g.drand(0.0, delta);
-      norm = sqrt(r2[0] * r2[0] + r2[1] * r2[1] + r2[2] * r2[2] + r2[3] * r2[3] + r2[4] * r2[4] + r2[5] * r2[5]);
-      if (T(1) != (T(1) + norm)) break;
-    }
-    fact = T(1) / norm;
-    z2[0] = fact * mk<T>(r2[0], r2[1]);
-    z2[1] = fact * mk<T>(r2[2], r2[3]);
-    z2[2] = fact * mk<T>(r2[4], r2[5]);
-    z = conj(z1[0]) * z2[0] + conj(z1[1]) * z2[1] + conj(z1[2]) * z2[2];
-    z2[0] -= z * z1[0];
-    z2[1] -= z * z1[1];
-    z2[2] -= z * z1[2];
-    norm = sqrt(z2[0].re * z2[0].re + z2[0].im * z2[0].im + z2[1].re * z2[1].re + z2[1].im * z2[1].im +
-                z2[2].re * z2[2].re + z2[2].im * z2[2].im);
-    if (T(1) != (T(1) + norm)) break;
-  }
-  fact = T(1) / norm;
-  z2[0] = z2[0] * fact;
-  z2[1] = z2[1] * fact;
-  z2[2] = z2[2] * fact;
+  for (int i = 0; i < 6; ++i) v[i] = (T)drand_u(0.0, delta, next());
+  norm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
+  return T(1) != (T(1) + norm);
+}
+template <typename T> KLFT_D void su3_row1(const T v[6], T norm, cx<T> z1[3]) {
+  const T fact = T(1) / norm;
+  z1[0] = fact * mk<T>(v[0], v[1]);
+  z1[1] = fact * mk<T>(v[2], v[3]);
+  z1[2] = fact * mk<T>(v[4], v[5]);
+}
+// z2 orthogonal to z1, its norm before normalisation returned
+template <typename T> KLFT_D T su3_row2(const T v[6], T n, const cx<T> z1[3], cx<T> z2[3]) {
+  su3_row1(v, n, z2);
+  const cx<T> z = conj(z1[0]) * z2[0] + conj(z1[1]) * z2[1] + conj(z1[2]) * z2[2];
+  z2[0] -= z * z1[0];
+  z2[1] -= z * z1[1];
+  z2[2] -= z * z1[2];
+  return sqrt(z2[0].re * z2[0].re + z2[0].im * z2[0].im + z2[1].re * z2[1].re + z2[1].im * z2[1].im +
+              z2[2].re * z2[2].re + z2[2].im * z2[2].im);
+}
+template <typename T> KLFT_D Mat<3, T> su3_rows(const cx<T> z1[3], const cx<T> z2in[3], T norm) {
+  const T fact = T(1) / norm;
+  cx<T> z2[3], z3[3];
+  z2[0] = z2in[0] * fact;
+  z2[1] = z2in[1] * fact;
+  z2[2] = z2in[2] * fact;
   z3[0] = conj((z1[1] * z2[2]) - (z1[2] * z2[1]));
   z3[1] = conj((z1[2] * z2[0]) - (z1[0] * z2[2]));
   z3[2] = conj((z1[0] * z2[1]) - (z1[1] * z2[0]));
+  Mat<3, T> r;
 #pragma unroll
   for (int j = 0; j < 3; ++j) { r.e[0][j] = z1[j]; r.e[1][j] = z2[j]; r.e[2][j] = z3[j]; }
   return r;
+}
+template <typename T, typename Next> KLFT_D bool su3_propose(Next &next, double delta, Mat<3, T> &r) {
+  T v[6], norm;
+  cx<T> z1[3], z2[3];
+  bool ok = su3_vec<T>(next, delta, v, norm);
+  su3_row1(v, norm, z1);
+  ok = su3_vec<T>(next, delta, v, norm) && ok;
+  norm = su3_row2(v, norm, z1, z2);
+  ok = ok && T(1) != (T(1) + norm);
+  r = su3_rows(z1, z2, norm);
+  return ok;
+}
+// The reference's redraws, in stream order (probability near 1e-16 per hit).
+// They are bounded here (the host rejects delta <= 0, for which they never end).
+template <typename T> __device__ __noinline__ void su3_propose_redraw(Stream &g, double delta, Mat<3, T> &r) {
+  auto next = [&] { return g.next(); };
+  T v[6], norm = T(0);
+  cx<T> z1[3], z2[3];
+  for (int tries = 0; tries < 64; ++tries)
+    if (su3_vec<T>(next, delta, v, norm)) break;
+  su3_row1(v, norm, z1);
+  for (int outer = 0; outer < 64; ++outer) {
+    for (int tries = 0; tries < 64; ++tries)
+      if (su3_vec<T>(next, delta, v, norm)) break;
+    norm = su3_row2(v, norm, z1, z2);
+    if (T(1) != (T(1) + norm)) break;
+  }
+  r = su3_rows(z1, z2, norm);
 }
 
 // ------------------------------------------------------------------ hot start

@@ -67,13 +67,103 @@ KLFT_D Site pass_site(const Geom &g, long long t, int val, int nd) {
 template <typename T> struct MinBlocks { static constexpr int v = 4; };
 template <> struct MinBlocks<double> { static constexpr int v = 2; };
 
-// Reference proposals: sequential per-site stream, exactly as the reference consumes it.
+// min(1, exp(-dS)) against the uniform u, for dS >= 0 (or NaN): u < exp(-dS) with
+// the exponential of T.  The fast exponential (relative error below 1e-5 for
+// dS < 80) decides unless u lies within 1e-4 of it, so the decision is always
+// that of the accurate one, which about one hit in 10^4 evaluates.
+template <typename T> KLFT_D bool accept_uniform(T dS, double u) {
+  if (dS < T(80)) {
+    const float e = __expf(-(float)dS), uf = (float)u;
+    if (uf < e * 0.9999f) return true;
+    if (uf > e * 1.0001f) return false;
+  }
+  return u < (double)exp(-dS);
+}
+
+// The uniforms of a site's reference stream, hit by hit.  A hit reads
+// RefDraws<NC>::n uniforms for its proposal and one more unless dS < 0, so the
+// lanes of a warp fall out of step in the stream.  With a sequential reader every
+// draw then runs the Philox rounds for some lane (U(1) 2, SU(2) 4, SU(3) 13
+// evaluations per hit); here each hit evaluates the blocks that can hold its
+// uniforms (1, 2, 7), all lanes together, and each lane selects by the parity of
+// its position, keeping the one uniform of the last block that the next hit may
+// still read.
+template <int NC> struct HitDraws {
+  static constexpr int K = RefDraws<NC>::n;
+  SiteStream st;
+  uint32_t pos = 0;   // next uniform of the stream
+  uint32_t used = 0;  // uniforms of the last proposal
+  double carry = 0.0;
+  KLFT_D explicit HitDraws(const SiteStream &s) : st(s) {}
+
+  // the proposal of the next hit and the uniform after it
+  template <typename T> KLFT_D Mat<NC, T> propose_next(double delta, double &uacc) {
+    const uint32_t blk = (pos + 1u) >> 1;
+    const bool odd = pos & 1u;
+    if constexpr (NC == 1) {
+      double a, b;
+      st.block(blk, a, b);
+      const double u[1] = {odd ? carry : a};
+      uacc = odd ? a : b;
+      carry = b;
+      used = 1u;
+      return propose<T>(u, delta, (const Mat<1, T> *)nullptr);
+    } else if constexpr (NC == 2) {
+      double a, b, c, d;
+      st.block(blk, a, b);
+      st.block(blk + 1u, c, d);
+      const double u[3] = {odd ? carry : a, odd ? a : b, odd ? b : c};
+      uacc = odd ? c : d;
+      carry = d;
+      used = 3u;
+      return propose<T>(u, delta, (const Mat<2, T> *)nullptr);
+    } else {
+      int i = 0;
+      double prev = carry, hi = 0.0;
+      auto next = [&] {
+        double w = hi;
+        if ((i & 1) == 0) st.block(blk + (uint32_t)(i >> 1), w, hi);
+        const double r = odd ? prev : w;
+        prev = w;
+        ++i;
+        return r;
+      };
+      Mat<3, T> r;
+      const bool ok = su3_propose<T>(next, delta, r);
+      uacc = next();
+      carry = odd ? uacc : hi;
+      used = 12u;
+      if (!ok) redraw<T>(delta, r, uacc);
+      return r;
+    }
+  }
+  // after the hit: drawn = the accept uniform was read
+  KLFT_D void advance(bool drawn) {
+    pos += used + (drawn ? 1u : 0u);
+    if constexpr (NC == 3) {
+      if (used != 12u && (pos & 1u)) {
+        double a;
+        st.block(pos >> 1, a, carry);
+      }
+    }
+  }
+
+ private:
+  template <typename T> KLFT_D void redraw(double delta, Mat<3, T> &r, double &uacc) {
+    Stream g = st.stream();
+    g.seek(pos);
+    su3_propose_redraw<T>(g, delta, r);
+    used = g.position() - pos;
+    uacc = g.next();
+  }
+};
+
 // The hits of link U_mu(x) in the reference's order (Metropolis.hpp:85-107),
-// drawing from the site's stream rng.  MU >= 0: mu at compile time (the staple's
+// drawing from the site's stream.  MU >= 0: mu at compile time (the staple's
 // site steps compiled, its nu loops unrolled); MU = -1: run-time mu.
 template <int NC, int ND, typename T, bool DF, int MU>
 KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, int mu, const MetroArgs &a,
-                           const Defect &df, Stream &rng, long long lx, T bnc) {
+                           const Defect &df, HitDraws<NC> &rng, long long lx, T bnc) {
   if (open_link(g, x, mu)) return 0;
   int nacc = 0;
   Mat<NC, T> S;
@@ -94,13 +184,15 @@ KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
     bool changed = false;
 #pragma unroll 1
     for (int hit = 0; hit < a.nhits; ++hit) {
-      const Mat<NC, T> rr = propose<T>(rng, (const Mat<NC, T> *)nullptr, a.delta, PROPOSAL_REFERENCE, 0.0);
+      double u;
+      const Mat<NC, T> rr = rng.template propose_next<T>(a.delta, u);
       const Mat<NC, T> Y = hit == 0 ? rr : mul(A, rr);
       const T tY = retr_mul(Y, M0);
       T dS = -bnc * (tY - trO);
       if (dlink) dS *= (T)defect_c(df);
-      bool accept = dS < T(0);
-      if (!accept) accept = rng.next() < (double)exp(-dS);
+      const bool down = dS < T(0);
+      const bool accept = down || accept_uniform(dS, u);
+      rng.advance(!down);
       if (accept) {
         A = Y;
         trO = tY;
@@ -117,11 +209,13 @@ KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
   bool changed = false;
 #pragma unroll 1
   for (int hit = 0; hit < a.nhits; ++hit) {
-    const Mat<NC, T> rr = propose<T>(rng, (const Mat<NC, T> *)nullptr, a.delta, PROPOSAL_REFERENCE, 0.0);
+    double u;
+    const Mat<NC, T> rr = rng.template propose_next<T>(a.delta, u);
     T dS = -bnc * (retr_mul(rr, M) - trO);
     if (dlink) dS *= (T)defect_c(df);
-    bool accept = dS < T(0);
-    if (!accept) accept = rng.next() < (double)exp(-dS);
+    const bool down = dS < T(0);
+    const bool accept = down || accept_uniform(dS, u);
+    rng.advance(!down);
     if (accept) {
       Uo = restore(mul(Uo, rr));
       M = mul(S, Uo);
@@ -138,7 +232,7 @@ template <int NC, int ND, typename T, bool DF>
 KLFT_D int site_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, const MetroArgs &a, uint32_t sweep,
                            const Defect &df) {
   int nacc = 0;
-  Stream rng(a.seed, a.chain, site_lex(g, x), sweep, KIND_METROPOLIS, 0);
+  HitDraws<NC> rng(SiteStream(a.seed, a.chain, site_lex(g, x), sweep, KIND_METROPOLIS));
   const long long lx = site_lin(g, x);
   const T bnc = (T)a.beta / (T)NC;
   if constexpr (NC <= 2 && !DF) {
