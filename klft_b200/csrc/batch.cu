@@ -24,41 +24,14 @@
 
 #include "../../include/klft_b200.h"
 #include "capi_internal.h"
+#include "chains.cuh"
 #include "kernels.cuh"
+#include "metropolis_group.cuh"
 #include "metropolis_site.cuh"
 #include "observables.cuh"
 #include "tuner.h"
 
 namespace klft {
-
-constexpr int BATCH_MAX = 64;
-
-struct ChainDesc {
-  void *links;
-  uint32_t *ctr;  // the chain's counters ([0] = sweep)
-  Geom g;
-  MetroArgs a;
-  Defect df;
-  int index;        // chain id in the batch
-  int block_begin;  // first CTA of this chain in the launch
-};
-
-struct ChainTable {
-  int n;
-  int nchains_total;
-  int block;  // threads per CTA of the launch (<= 128)
-  ChainDesc c[BATCH_MAX];
-};
-
-KLFT_D int find_chain(const ChainTable &tab) {
-  int lo = 0, hi = tab.n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tab.c[mid].block_begin <= (int)blockIdx.x) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
 
 // MU >= 0 (exp groups): the link pass's direction at compile time (val >> 1 == MU)
 template <int NC, int ND, typename T, bool EXP, bool DF, int MU = -1>
@@ -337,8 +310,21 @@ cudaError_t launch_group_nc(const GroupKey &k, const ChainTable &tab, int blocks
   return launch_group_nd<NC, 4, T>(k, tab, blocks, val, nacc, slot, st);
 }
 
-cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, int val, unsigned long long *nacc,
-                         const uint32_t *slot, cudaStream_t st) {
+// lanes > 1: the reference-proposal pass by groups of lanes (metropolis_group.cuh)
+cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, int lanes, int val,
+                         unsigned long long *nacc, const uint32_t *slot, cudaStream_t st) {
+  if (lanes > 1) {
+    GroupLaunch l;
+    l.tab = &tab;
+    l.blocks = blocks;
+    l.slot = slot;
+    l.val = val;
+    l.nacc = nacc;
+    l.st = st;
+    if (k.nc == 1) return launch_group_u1(k.nd, k.dtype, lanes, k.df, l);
+    if (k.nc == 2) return launch_group_su2(k.nd, k.dtype, lanes, k.df, l);
+    return launch_group_su3(k.nd, k.dtype, lanes, k.df, l);
+  }
   if (k.dtype == 0) {
     if (k.nc == 1) return launch_group_nc<1, double>(k, tab, blocks, val, nacc, slot, st);
     if (k.nc == 2) return launch_group_nc<2, double>(k, tab, blocks, val, nacc, slot, st);
@@ -351,9 +337,16 @@ cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, i
 
 struct Group {
   GroupKey key;
+  long long sites = 0;  // of one pass, all chains
+  int lanes = 1;        // per site (reference proposals)
   std::vector<std::unique_ptr<ChainTable>> tables;
   std::vector<int> blocks;
 };
+
+GroupKey key_of(const klft::SweepItem &it) {
+  return GroupKey{it.lat->nc, it.lat->g.nd, it.lat->dtype(),
+                  (it.lat->nc == 3 && it.a.proposal == KLFT_PROPOSAL_EXP) ? 1 : 0, it.df.active ? 1 : 0};
+}
 
 }  // namespace
 
@@ -369,18 +362,21 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
   const int n = (int)items.size();
   const int stride = acc_stride > 0 ? acc_stride : n;
   std::vector<Group> groups;
+  auto group_of = [&](const GroupKey &key) -> Group & {
+    for (auto &gg : groups)
+      if (gg.key == key) return gg;
+    groups.emplace_back();
+    groups.back().key = key;
+    return groups.back();
+  };
+  for (const SweepItem &it : items) group_of(key_of(it)).sites += it.lat->g.Vh;
+  for (auto &gg : groups)
+    if (!gg.key.exp) gg.lanes = group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
   for (int i = 0; i < n; ++i) {
     const SweepItem &it = items[i];
     klft_lattice *lat = it.lat;
-    GroupKey key{lat->nc, lat->g.nd, lat->dtype(), (lat->nc == 3 && it.a.proposal == KLFT_PROPOSAL_EXP) ? 1 : 0,
-                 it.df.active ? 1 : 0};
-    Group *grp = nullptr;
-    for (auto &gg : groups)
-      if (gg.key == key) grp = &gg;
-    if (!grp) {
-      groups.push_back(Group{key, {}, {}});
-      grp = &groups.back();
-    }
+    const GroupKey key = key_of(it);
+    Group *grp = &group_of(key);
     if (grp->tables.empty() || grp->tables.back()->n == BATCH_MAX) {
       grp->tables.emplace_back(new ChainTable());
       std::memset(grp->tables.back().get(), 0, sizeof(ChainTable));
@@ -401,7 +397,7 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
     d.block_begin = grp->blocks.back();
     // exp groups: V/2 links per link pass; reference groups: Vh sites per class
     const long long nthr = key.exp ? link_pass_threads(lat->g, lat->g.nd) : lat->g.Vh;
-    grp->blocks.back() += (int)((nthr + block - 1) / block);
+    grp->blocks.back() += grp->lanes > 1 ? (int)group_blocks(lat->g.Vh, grp->lanes) : (int)((nthr + block - 1) / block);
   }
   int maxpass = 0;
   for (auto &gg : groups) {
@@ -422,7 +418,7 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
       if (val >= (gg.key.exp ? 2 * gg.key.nd : 1 << gg.key.nd)) continue;
       const cudaStream_t gs = gi == 0 || nside == 0 ? st : fork->side[(gi - 1) % nside];
       for (size_t t = 0; t < gg.tables.size() && err == cudaSuccess; ++t) {
-        err = launch_group(gg.key, *gg.tables[t], gg.blocks[t], val, nacc, slot, gs);
+        err = launch_group(gg.key, *gg.tables[t], gg.blocks[t], gg.lanes, val, nacc, slot, gs);
         if (nlaunch) ++*nlaunch;
       }
     }

@@ -22,6 +22,12 @@ const double *bm_table();
 // (proposal 1), else the reference's 2^Nd site classes.
 KLFT_HD int metropolis_passes(int nc, int proposal, int nd) { return nc == 3 && proposal == 1 ? 2 * nd : 1 << nd; }
 
+// Reference proposals: lanes per site of a pass over `sites` sites (all chains of a
+// launch), 1 = one thread per site (site_update_ref), else metropolis_group.cuh.
+int group_lanes(int nc, int dtype, bool defect, long long sites);
+constexpr int GROUP_THREADS = 64;  // per CTA of the group kernels: few sites over many SMs
+inline long long group_blocks(long long sites, int lanes) { return (sites * lanes + GROUP_THREADS - 1) / GROUP_THREADS; }
+
 // dtype: 0 = double (plain FP64 form), 1 = float (mixed form)
 // val: the site class, or the link pass 2 mu + parity of the exp proposal
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,

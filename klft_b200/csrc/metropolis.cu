@@ -7,7 +7,7 @@
 // a pass is race free.  exp(i eps H) proposals: 2 Nd link passes (mu, parity)
 // of one thread per link (metropolis_site.cuh).  The per-site and per-link
 // updates are in metropolis_site.cuh.
-#include "metropolis_site.cuh"
+#include "metropolis_group.cuh"
 
 namespace klft {
 
@@ -85,9 +85,43 @@ static cudaError_t launch_nd(int nd, void *links, const Geom &g, int val, const 
   return cudaErrorInvalidValue;
 }
 
+// More lanes shorten a site's chain of proposals but repeat its serial part in every
+// lane and form proposals that are not used, so they pay while the sites leave the
+// device idle.  us per sweep (4-D, nHits 10, FP64 | FP32), one thread per site
+// against a group:
+//   U(1)   8^4 497|463 -> 32 lanes 180|155, 12x8x10x20 497|466 -> 208|207,
+//          16^4 497|470 -> 16 lanes 368|286 (32: 450|412), 16^3x32 497|481, 16 lanes 652|558
+//   SU(2)  8^4 824|530 -> 32 lanes 241|200, 12x8x10x20 825|534 -> 370|285,
+//          16^4 824|535 -> 16 lanes 725|465 (32: 746|577), 16^3x32 824|535, 16 lanes 1347|890
+//   SU(3)  8^4 1259|1382 -> 32 lanes 199|175, 12x8x10x20 1260|1388 -> 8 lanes 350|307
+//          (32: 440|268), 16^4 1259|1382 -> 499|443, 16^3x32 1265|1382 -> 973|781,
+//          24^4 1716|1647, 8 lanes 2219|1369
+// A pass has V / 16 sites: 256, 1200, 4096, 8192, 20736.
+int group_lanes(int nc, int dtype, bool defect, long long sites) {
+  if (nc == 3) return sites <= 800 ? 32 : (sites <= (dtype == 0 ? 12000 : 24000) ? 8 : 1);
+  if (defect && dtype == 1) return 1;  // no FP32 form for U(1), SU(2) with a defect
+  return sites <= 2048 ? 32 : (sites <= 5000 ? 16 : 1);
+}
+
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,
                                    const uint32_t *d_sweep, unsigned long long *d_nacc, const Defect &df, int block,
                                    cudaStream_t st) {
+  const bool exp = nc == 3 && a.proposal == PROPOSAL_EXP;
+  const int lanes = exp ? 1 : group_lanes(nc, dtype, df.active != 0, g.Vh);
+  if (lanes > 1) {
+    GroupLaunch l;
+    l.links = links;
+    l.g = &g;
+    l.a = &a;
+    l.df = &df;
+    l.d_sweep = d_sweep;
+    l.val = val;
+    l.nacc = d_nacc;
+    l.st = st;
+    if (nc == 1) return launch_group_u1(g.nd, dtype, lanes, df.active != 0, l);
+    if (nc == 2) return launch_group_su2(g.nd, dtype, lanes, df.active != 0, l);
+    return launch_group_su3(g.nd, dtype, lanes, df.active != 0, l);
+  }
   if (dtype == 0) {
     if (nc == 3 && a.proposal == 1) {
       // the FP64 exp(i eps H) proposal reads its Gaussians from the host-built table

@@ -1,0 +1,609 @@
+// metropolis_group.cuh -- the reference-proposal update of one site by a group of
+// G lanes, for passes with too few sites to fill the device with one thread each.
+//
+// site_update_ref runs a site's Nd links and their hits one after another in one
+// thread: Nd * nhits proposals (Philox rounds, sine and cosine, norms), each on
+// the chain of the one before, and Nd staples whose loads wait for each other.  A
+// class of 8^4 has 256 sites, so that chain is the whole pass.  Only two things
+// in it are sequential: the accept decisions and the place in the site's stream
+// they leave it at.  The lanes of a group share the rest:
+//
+//  * U(1), SU(2): the lanes form the uniforms of a window of the stream and the
+//    proposal that would start at each place in it; a hit then takes the one at
+//    its place.  Most are not used (a hit moves on by 1-2 or 3-4 places).  The
+//    links around the site are brought into L1 by all lanes at once, then every
+//    lane runs link_update_ref.
+//  * SU(3), where a few per cent of the hits are accepted: lane j forms the
+//    proposal and the action change of the j-th hit from here, as if every hit
+//    before it were rejected with its uniform drawn; the group keeps the hits
+//    before the first exception, applies that one and goes on from there.  The
+//    products of neighbour links in the staples of all directions are shared out
+//    as well: links of one class are not neighbours, so only U_nu(x) itself
+//    changes while the site is updated.
+//
+// None of the proposals read links, so the first ones come before the wait for
+// the pass before (programmatic dependent launch).  Operations on a link and
+// their order are those of site_update_ref; the chain is the same.
+#pragma once
+#include "chains.cuh"
+#include "metropolis_site.cuh"
+
+namespace klft {
+
+KLFT_D void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+KLFT_D void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <int G> KLFT_D unsigned group_mask() {
+  if constexpr (G == 32) return 0xffffffffu;
+  else return ((1u << G) - 1u) << (threadIdx.x & 31u & ~(unsigned)(G - 1));
+}
+
+// ------------------------------------------------------------------ U(1), SU(2)
+// Window of stream places in shared memory, per group.
+template <int NC, typename T, int G> struct DrawTable {
+  static constexpr int K = RefDraws<NC>::n;
+  static constexpr int W = G == 32 ? (NC == 1 ? 96 : 160) : 32;
+  static constexpr int N = W + K + 2;  // a hit looks up to K + 1 places past its own
+  cx<T> prop[N][NC];  // row 0 of the proposal starting at each place
+  double u[N];
+  float lg[N];  // ln u (NaN for u = 0)
+};
+
+// HitDraws for a group: the same uniforms and proposals, from the group's table.
+template <int NC, typename T, int G> struct TableDraws {
+  using Table = DrawTable<NC, T, G>;
+  static constexpr int K = Table::K;
+  Table &tab;
+  const SiteStream st;
+  const double delta;
+  long long left;       // hits that may still come
+  const int gl;         // lane in the group
+  const unsigned mask;  // the group's lanes
+  int wn = 0, i = 0;    // window: places [base, base + wn) of the stream; the next hit's place
+  uint32_t base = 0;
+  bool have = false;
+  cx<T> r[NC], ra[NC], rb[NC];  // row 0 of this hit's proposal, of the two that can come next
+  float lg = 0.f, la = 0.f, lb = 0.f;
+
+  KLFT_D TableDraws(Table &t, const SiteStream &s, double delta_, long long hits)
+      : tab(t), st(s), delta(delta_), left(hits), gl((int)(threadIdx.x & (unsigned)(G - 1))), mask(group_mask<G>()) {}
+
+  // the window from the next hit's place on
+  KLFT_D void fill() {
+    __syncwarp(mask);
+    const uint32_t pos = base + (uint32_t)i;
+    base = pos & ~1u;
+    i = (int)(pos & 1u);
+    const long long need = (left * (K + 1) + i + 1) & ~1ll;
+    wn = need < Table::W ? (int)need : Table::W;
+    for (int b = gl; 2 * b < wn; b += G) {
+      double u0, u1;
+      st.block((base >> 1) + (uint32_t)b, u0, u1);
+      tab.u[2 * b] = u0;
+      tab.u[2 * b + 1] = u1;
+      tab.lg[2 * b] = u0 > 0.0 ? __logf((float)u0) : __int_as_float(0x7fc00000);
+      tab.lg[2 * b + 1] = u1 > 0.0 ? __logf((float)u1) : __int_as_float(0x7fc00000);
+    }
+    __syncwarp(mask);
+    for (int p = gl; p + K < wn; p += G) {
+      const Mat<NC, T> m = propose<T>(&tab.u[p], delta, (const Mat<NC, T> *)nullptr);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) tab.prop[p][j] = m.e[0][j];
+    }
+    __syncwarp(mask);
+    have = false;
+  }
+
+  template <typename> KLFT_D Mat<NC, T> propose_next(double, double &) {
+    if (i + K >= wn) fill();
+    if (!have) {
+#pragma unroll
+      for (int j = 0; j < NC; ++j) r[j] = tab.prop[i][j];
+      lg = tab.lg[i + K];
+      have = true;
+    }
+    // both places the next hit can be at, loaded beside this hit's arithmetic
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      ra[j] = tab.prop[i + K][j];
+      rb[j] = tab.prop[i + K + 1][j];
+    }
+    la = tab.lg[i + 2 * K];
+    lb = tab.lg[i + 2 * K + 1];
+    --left;
+    Mat<NC, T> m;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) m.e[0][j] = r[j];
+    if constexpr (NC == 2) su2_row1(m);
+    return m;
+  }
+  // u < exp(-dS) from ln u <= 0 in FP32 (absolute error below 2e-5); within 1e-4, and
+  // for u = 0 or a NaN, the accurate comparison of accept_uniform
+  KLFT_D bool accept(T dS, double) const {
+    const float t = (float)dS + lg;
+    if (fabsf(t) > 1e-4f) return t < 0.f;
+    return tab.u[i + K] < (double)exp(-dS);
+  }
+  KLFT_D void advance(bool drawn) {
+    i += drawn ? K + 1 : K;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) r[j] = drawn ? rb[j] : ra[j];
+    lg = drawn ? lb : la;
+  }
+};
+
+// One lane's share of the links that the staples of site x read, into L1.
+template <int NC, int ND, typename T, int G>
+KLFT_D void touch_neighbours(const Links<NC, T> &U, const Geom &g, const Site &x, int gl) {
+  // q = (mu, nu): U_mu(x-nu) always, U_nu(x+mu) and U_nu(x+mu-nu) for nu != mu
+  for (int q = gl; q < ND * ND; q += G) {
+    const int mu = q / ND, nu = q - mu * ND;
+    const Site xp = site_up(g, x, mu);
+    const long long lin[3] = {site_lin(g, site_dn(g, x, nu)), site_lin(g, xp), site_lin(g, site_dn(g, xp, nu))};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (k > 0 && mu == nu) break;
+      const cx<T> *p = U.p + (long long)(k == 0 ? mu : nu) * Links<NC, T>::P * U.V + lin[k];
+#pragma unroll
+      for (int c = 0; c < Links<NC, T>::P; ++c) {
+        float d;  // the value is not used: nothing waits for the load
+        asm volatile("ld.global.ca.f32 %0, [%1];" : "=f"(d) : "l"(p + c * U.V) : "memory");
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ U(1), SU(2) in FP64
+// The hits of a link with staple S, as in link_update_ref; Uo: the link, updated when
+// any is accepted.
+template <int NC, typename T, typename Draws>
+KLFT_D int group_hits(const Mat<NC, T> &S, Mat<NC, T> &Uo, const MetroArgs &a, bool dlink, const Defect &df,
+                      Draws &rng, T bnc) {
+  const Mat<NC, T> U0 = Uo, M0 = mul(S, U0);
+  const T cdef = dlink ? (T)defect_c(df) : T(1);
+  Mat<NC, T> A = mident<NC, T>();
+  T trO = retr_diag(M0);
+  int nacc = 0;
+#pragma unroll 1
+  for (int hit = 0; hit < a.nhits; ++hit) {
+    double u;
+    const Mat<NC, T> Y = mul(A, rng.template propose_next<T>(a.delta, u));
+    const T tY = retr_mul(Y, M0);
+    const T dS = -bnc * (tY - trO) * cdef;
+    const bool down = dS < T(0);
+    const bool accept = down || rng.accept(dS, u);
+    rng.advance(!down);
+    if (accept) {
+      A = Y;
+      trO = tY;
+      ++nacc;
+    }
+  }
+  if (nacc) Uo = restore(mul(U0, A));
+  return nacc;
+}
+
+// ------------------------------------------------------------------ U(1), SU(2) in FP32
+// link_update_ref for a group, its products with their FMAs written out: the
+// compiler contracts a b + c d by the order in which it finds the operands, which
+// here is another one, and the FP32 chain is to be bit for bit the one of
+// site_update_ref (its accept decisions turn on the last bit).  Each form below is
+// the one that agrees with that function over 10^9 hits in 2, 3 and 4 dimensions.
+KLFT_D float mad2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }  // a b + c d
+
+template <int NC> struct Row0 { cx<float> v[NC]; };  // SU(2): row 0 of the matrix
+template <int NC> KLFT_D Row0<NC> row0(const Mat<NC, float> &m) {
+  Row0<NC> r;
+#pragma unroll
+  for (int j = 0; j < NC; ++j) r.v[j] = m.e[0][j];
+  return r;
+}
+// S U0
+KLFT_D Row0<1> group_mul_link(const Row0<1> &s, const Row0<1> &u) {
+  const cx<float> a = s.v[0], b = u.v[0];
+  return {{mk<float>(mad2(a.re, b.re, -a.im, b.im), mad2(a.im, b.re, a.re, b.im))}};
+}
+KLFT_D float su2_re00(const Row0<2> &x, const Row0<2> &y) {
+  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
+  return __fadd_rn(mad2(a.re, c.re, -a.im, c.im), mad2(b.re, -d.re, -b.im, d.im));
+}
+KLFT_D Row0<2> group_mul_link(const Row0<2> &s, const Row0<2> &u) {
+  const cx<float> a = s.v[0], b = s.v[1], c = u.v[0], d = u.v[1];
+  return {{mk<float>(su2_re00(s, u), __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.re, d.im, b.im, -d.re))),
+           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im)),
+                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
+}
+// A r
+KLFT_D Row0<1> group_mul_hit(const Row0<1> &x, const Row0<1> &r) { return group_mul_link(x, r); }
+KLFT_D Row0<2> group_mul_hit(const Row0<2> &x, const Row0<2> &r) {
+  const cx<float> a = x.v[0], b = x.v[1], c = r.v[0], d = r.v[1];
+  return {{mk<float>(su2_re00(x, r), __fadd_rn(mad2(a.re, c.im, a.im, c.re), mad2(b.re, d.im, b.im, -d.re))),
+           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.im, c.im, b.re, c.re)),
+                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
+}
+// Re Tr(Y M0)
+KLFT_D float group_retr(const Row0<1> &y, const Row0<1> &m) {
+  return mad2(y.v[0].re, m.v[0].re, -y.v[0].im, m.v[0].im);
+}
+KLFT_D float group_retr(const Row0<2> &y, const Row0<2> &m) {
+  const cx<float> a = y.v[0], b = y.v[1], c = m.v[0], d = m.v[1];
+  const float h = __fadd_rn(mad2(-a.im, c.im, a.re, c.re), mad2(b.re, -d.re, -b.im, d.im));
+  return __fadd_rn(h, h);
+}
+KLFT_D float group_retr(const Row0<1> &m) { return m.v[0].re; }
+KLFT_D float group_retr(const Row0<2> &m) { return __fadd_rn(m.v[0].re, m.v[0].re); }
+// restore(U0 A); FIRST: direction 0
+template <bool FIRST> KLFT_D Row0<1> group_new_link(const Row0<1> &u, const Row0<1> &x) {
+  const cx<float> a = u.v[0], c = x.v[0];
+  const float re = mad2(a.re, c.re, -a.im, c.im);
+  const float im = FIRST ? mad2(a.re, c.im, a.im, c.re) : mad2(a.im, c.re, a.re, c.im);
+  const float i = 1.0f / sqrtf(mad2(re, re, im, im));
+  return {{mk<float>(__fmul_rn(re, i), __fmul_rn(im, i))}};
+}
+template <bool FIRST> KLFT_D Row0<2> group_new_link(const Row0<2> &u, const Row0<2> &x) {
+  const cx<float> a = u.v[0], b = u.v[1], c = x.v[0], d = x.v[1];
+  cx<float> p, q;
+  p.re = su2_re00(u, x);
+  q.re = __fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im));
+  if constexpr (FIRST) {
+    p.im = __fadd_rn(mad2(a.re, c.im, a.im, c.re), mad2(b.re, d.im, b.im, -d.re));
+    q.im = __fadd_rn(mad2(a.re, d.im, a.im, d.re), mad2(b.re, -c.im, b.im, c.re));
+  } else {
+    p.im = __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.im, -d.re, b.re, d.im));
+    q.im = __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im));
+  }
+  const float i = 1.0f / sqrtf(fmaf(q.im, q.im, fmaf(q.re, q.re, mad2(p.re, p.re, p.im, p.im))));
+  return {{mk<float>(__fmul_rn(p.re, i), __fmul_rn(p.im, i)), mk<float>(__fmul_rn(q.re, i), __fmul_rn(q.im, i))}};
+}
+template <int NC, int ND, int MU, typename Draws>
+KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &x, const MetroArgs &a, Draws &rng) {
+  if constexpr (MU < ND) {
+    if (open_link(g, x, MU)) return 0;
+    const long long lx = site_lin(g, x);
+    const float bnc = (float)a.beta / (float)NC;
+    const Row0<NC> S = row0(staple_ct<NC, ND, MU, float>(U, g, x)), U0 = row0(U.load(lx, MU));
+    const Row0<NC> M0 = group_mul_link(S, U0);
+    Row0<NC> A = row0(mident<NC, float>());
+    float trO = group_retr(M0);
+    int nacc = 0;
+#pragma unroll 1
+    for (int hit = 0; hit < a.nhits; ++hit) {
+      double u;
+      const Row0<NC> Y = group_mul_hit(A, row0(rng.template propose_next<float>(a.delta, u)));
+      const float tY = group_retr(Y, M0);
+      const float dS = __fmul_rn(-bnc, __fsub_rn(tY, trO));
+      const bool down = dS < 0.f;
+      const bool accept = down || rng.accept(dS, u);
+      rng.advance(!down);
+      if (accept) {
+        A = Y;
+        trO = tY;
+        ++nacc;
+      }
+    }
+    if (nacc) {
+      const Row0<NC> V = group_new_link<MU == 0>(U0, A);
+      Mat<NC, float> m;
+#pragma unroll
+      for (int j = 0; j < NC; ++j) m.e[0][j] = V.v[j];
+      U.store(lx, MU, m);
+    }
+    return nacc;
+  }
+  return 0;
+}
+
+// ------------------------------------------------------------------ staples shared out
+// m as Links::load returns it after Links::store(m)
+template <int NC, typename T> KLFT_D Mat<NC, T> as_stored(Mat<NC, T> m) {
+  if constexpr (LinkPlanes<NC, T>::n < NC * NC) {
+    if constexpr (NC == 3) complete_row2(m);
+    else su2_row1(m);
+  }
+  return m;
+}
+
+// The links of a site and the products of its neighbours' links, per group.
+template <int NC, int ND, typename T> struct StapleParts {
+  Mat<NC, T> own[ND];
+  // [mu][forward nu, backward nu]: U_nu(x+mu) U_mu(x+nu)^+, the whole backward term
+  Mat<NC, T> part[2 * ND * (ND - 1)];
+
+  template <bool DF, int G>
+  KLFT_D void load(const Links<NC, T> &U, const Geom &g, const Site &x, long long lx, const Defect &df, int gl) {
+    for (int d = gl; d < ND; d += G) own[d] = U.load(lx, d);
+    for (int q = gl; q < 2 * ND * (ND - 1); q += G) {
+      const int mu = q / (2 * (ND - 1)), r = q - mu * 2 * (ND - 1);  // r: forward, then backward nu
+      const bool fwd = r < ND - 1;
+      int nu = fwd ? r : r - (ND - 1);
+      nu += nu >= mu;
+      const Site xpmu = site_up(g, x, mu), xmnu = site_dn(g, x, nu);
+      // forward A B^+ = U_nu(x+mu) U_mu(x+nu)^+, backward D^+ E^+ G with
+      // D = U_nu(x+mu-nu), E = U_mu(x-nu), G = U_nu(x-nu)
+      const Mat<NC, T> a1 = load_link<NC, T, DF>(U, g, fwd ? xpmu : site_dn(g, xpmu, nu), nu, df);
+      const Mat<NC, T> a2 = load_link<NC, T, DF>(U, g, fwd ? site_up(g, x, nu) : xmnu, mu, df);
+      Mat<NC, T> t = mul_nd(fwd ? a1 : dagger(a1), a2);
+      if (!fwd) t = mul(t, load_link<NC, T, DF>(U, g, xmnu, nu, df));
+      part[q] = t;
+    }
+  }
+
+  // staple(): all forward terms, then all backward ones
+  template <bool DF> KLFT_D Mat<NC, T> staple(int mu, bool own0_in_defect, const Defect &df) const {
+    Mat<NC, T> S = mzero<NC, T>();
+    const Mat<NC, T> *p = part + mu * 2 * (ND - 1);
+#pragma unroll 1
+    for (int k = 0; k < ND - 1; ++k) {
+      const int nu = k + (k >= mu);
+      Mat<NC, T> c = own[nu];
+      if constexpr (DF) {
+        if (nu == 0 && own0_in_defect) c = mscale(c, (T)defect_c(df));
+      }
+      madd(S, mul_nd(p[k], c));
+    }
+#pragma unroll 1
+    for (int k = 0; k < ND - 1; ++k) madd(S, p[ND - 1 + k]);
+    return S;
+  }
+};
+
+// The links of site x in the order mu = 0 .. Nd-1 from shared parts; hits(S, U, dlink)
+// updates one link and returns its accepted hits, the same in every lane.
+template <int NC, int ND, typename T, bool DF, int G, typename Hits>
+KLFT_D int group_links(StapleParts<NC, ND, T> &sh, const Links<NC, T> &U, const Geom &g, const Site &x,
+                       const Defect &df, Hits &&hits) {
+  const long long lx = site_lin(g, x);
+  const int gl = (int)(threadIdx.x & (unsigned)(G - 1));
+  const unsigned mask = group_mask<G>();
+  sh.template load<DF, G>(U, g, x, lx, df, gl);
+  __syncwarp(mask);
+  const bool own0 = DF && df.active && in_defect(g, df, x, 0);
+  int nacc = 0;
+#pragma unroll 1
+  for (int mu = 0; mu < ND; ++mu) {
+    if (open_link(g, x, mu)) continue;
+    Mat<NC, T> V = sh.own[mu];
+    const int n = hits(sh.template staple<DF>(mu, own0, df), V, mu == 0 && own0);
+    if (n) {
+      __syncwarp(mask);
+      if (gl == 0) {
+        U.store(lx, mu, V);
+        sh.own[mu] = as_stored<NC, T>(V);
+      }
+      __syncwarp(mask);
+    }
+    nacc += n;
+  }
+  return nacc;
+}
+
+// ------------------------------------------------------------------ SU(3)
+// The hits of a site's links, one per lane.
+template <typename T, int G> struct LaneHits3 {
+  const MetroArgs &a;
+  const SiteStream st;
+  const int gl;         // lane in the group
+  const unsigned mask;  // the group's lanes
+  uint32_t pos = 0;     // place of the next hit in the stream
+  // this lane's hit of the chunk: proposal, the uniform after it, uniforms it took
+  Mat<3, T> rr;
+  double uacc = 0.0;
+  uint32_t used = 12u;
+  int ci = G;  // the chunk's next hit (G: none left)
+
+  KLFT_D LaneHits3(const MetroArgs &args, const SiteStream &stream)
+      : a(args), st(stream), gl((int)(threadIdx.x & (unsigned)(G - 1))), mask(group_mask<G>()) {}
+
+  // lane j: the proposal of the j-th hit from pos if no place is skipped
+  KLFT_D void chunk() {
+    HitDraws<3> d(st);
+    d.pos = pos + 13u * (uint32_t)gl;
+    if (d.pos & 1u) {
+      double u0;
+      st.block(d.pos >> 1, u0, d.carry);
+    }
+    rr = d.template propose_next<T>(a.delta, uacc);
+    used = d.used;
+    ci = 0;
+  }
+
+  // the hits of a link; Uo: the link, updated; the number accepted
+  KLFT_D int hits(const Mat<3, T> &S, Mat<3, T> &Uo, T bnc, bool dlink, T cdef) {
+    int nacc = 0;
+    Mat<3, T> M = mul(S, Uo);
+    T trO = retr_diag(M);
+    int hit = 0;
+    while (hit < a.nhits) {
+      if (ci == G) chunk();
+      const int n = a.nhits - hit < G - ci ? a.nhits - hit : G - ci;
+      const bool mine = gl >= ci && gl < ci + n;
+      bool down = false, accept = false;
+      if (mine) {
+        T dS = -bnc * (retr_mul(rr, M) - trO);
+        if (dlink) dS *= cdef;
+        down = dS < T(0);
+        accept = down || accept_uniform(dS, uacc);
+      }
+      const unsigned ev = __ballot_sync(mask, mine && (accept || down || used != 12u));
+      if (!ev) {
+        hit += n;
+        ci += n;
+        pos += 13u * (uint32_t)n;
+        continue;
+      }
+      const int src = __ffs((int)ev) - 1;  // lane of the warp
+      const int f = src & (G - 1);
+      const bool fdown = __shfl_sync(mask, down, src), facc = __shfl_sync(mask, accept, src);
+      const uint32_t fused = __shfl_sync(mask, used, src);
+      pos += 13u * (uint32_t)(f - ci);
+      hit += f - ci + 1;
+      if (facc) {
+        Mat<3, T> r;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            r.e[i][j].re = __shfl_sync(mask, rr.e[i][j].re, src);
+            r.e[i][j].im = __shfl_sync(mask, rr.e[i][j].im, src);
+          }
+        Uo = restore(mul(Uo, r));
+        M = mul(S, Uo);
+        trO = retr_diag(M);
+        ++nacc;
+      }
+      const uint32_t step = fused + (fdown ? 0u : 1u);
+      pos += step;
+      ci = step == 13u ? f + 1 : G;  // the chunk's later proposals hold unless the place moved
+    }
+    return nacc;
+  }
+};
+
+// ------------------------------------------------------------------ one site
+// Whether the staples are formed from shared parts.  In FP32 U(1) and SU(2) they
+// are not: their sums of two products are contracted by context too, so every lane
+// forms the staple as site_update_ref does, from links already in L1.
+template <int NC, typename T> struct SharedStaples { static constexpr bool v = NC == 3 || sizeof(T) == 8; };
+
+template <int NC, int ND, typename T, int G> struct GroupShared {
+  DrawTable<NC, T, G> table;
+  StapleParts<NC, SharedStaples<NC, T>::v ? ND : 1, T> parts;
+};
+template <int ND, typename T, int G> struct GroupShared<3, ND, T, G> { StapleParts<3, ND, T> parts; };
+
+// Site t (if t < Vh) of class val by the calling thread's group; sh: one entry per
+// group of the CTA.  Every thread of the CTA calls it and passes the wait.  The
+// sweep counter is read before it: a pass launched as a programmatic dependent
+// has only passes of its own sweep before it that may still run.  Accepted hits,
+// counted in one lane of the group.
+template <int NC, int ND, typename T, bool DF, int G>
+KLFT_D int group_site_update(GroupShared<NC, ND, T, G> *shared, const Links<NC, T> &U, const Geom &g, long long t, int val, const MetroArgs &a, uint32_t sweep, const Defect &df) {
+  const bool ok = t < g.Vh;
+  const Site x = pass_site(g, ok ? t : 0, val, ND);
+  const SiteStream st(a.seed, a.chain, site_lex(g, x), sweep, KIND_METROPOLIS);
+  GroupShared<NC, ND, T, G> &sh = shared[threadIdx.x / G];
+  const int gl = (int)(threadIdx.x & (unsigned)(G - 1));
+  const T bnc = (T)a.beta / (T)NC;
+  int n = 0;
+  if constexpr (NC == 3) {
+    LaneHits3<T, G> lanes(a, st);
+    if (ok) lanes.chunk();
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (ok)
+      n = group_links<3, ND, T, DF, G>(sh.parts, U, g, x, df, [&](const Mat<3, T> &S, Mat<3, T> &V, bool dlink) {
+        return lanes.hits(S, V, bnc, dlink, dlink ? (T)defect_c(df) : T(1));
+      });
+  } else {
+    TableDraws<NC, T, G> rng(sh.table, st, a.delta, (long long)ND * a.nhits);
+    if (ok) rng.fill();
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (ok) {
+      if constexpr (SharedStaples<NC, T>::v) {
+        n = group_links<NC, ND, T, DF, G>(sh.parts, U, g, x, df, [&](const Mat<NC, T> &S, Mat<NC, T> &V, bool dlink) {
+          return group_hits<NC, T>(S, V, a, dlink, df, rng, bnc);
+        });
+      } else {
+        // every lane: the same links, decisions and stores
+        static_assert(!DF, "FP32 U(1), SU(2): lattices without a defect");
+        touch_neighbours<NC, ND, T, G>(U, g, x, gl);
+        n = group_link_f32<NC, ND, 0>(U, g, x, a, rng);
+        n += group_link_f32<NC, ND, 1>(U, g, x, a, rng);
+        n += group_link_f32<NC, ND, 2>(U, g, x, a, rng);
+        n += group_link_f32<NC, ND, 3>(U, g, x, a, rng);
+      }
+    }
+  }
+  return gl == 0 ? n : 0;
+}
+
+// ------------------------------------------------------------------ kernels
+// the reference-proposal pass of one lattice
+template <int NC, int ND, typename T, bool DF, int G>
+__global__ void __launch_bounds__(GROUP_THREADS)
+    metropolis_group_kernel(Links<NC, T> U, Geom g, int val, MetroArgs a, const uint32_t *__restrict__ d_sweep,
+                            unsigned long long *__restrict__ d_nacc, Defect df) {
+  __shared__ GroupShared<NC, ND, T, G> sh[GROUP_THREADS / G];
+  const long long t = ((long long)blockIdx.x * GROUP_THREADS + threadIdx.x) / G;
+  add_accepts(group_site_update<NC, ND, T, DF, G>(sh, U, g, t, val, a, *d_sweep, df), d_nacc);
+}
+
+// the same pass of many chains (multi_pass_kernel)
+template <int NC, int ND, typename T, bool DF, int G>
+__global__ void __launch_bounds__(GROUP_THREADS)
+    multi_group_kernel(const __grid_constant__ ChainTable tab, int val, unsigned long long *nacc_slots,
+                       const uint32_t *__restrict__ slot) {
+  __shared__ GroupShared<NC, ND, T, G> sh[GROUP_THREADS / G];
+  const ChainDesc &c = tab.c[find_chain(tab)];
+  const long long t = ((long long)(blockIdx.x - c.block_begin) * GROUP_THREADS + threadIdx.x) / G;
+  const Links<NC, T> U{(cx<T> *)c.links, c.g.V};
+  add_accepts(group_site_update<NC, ND, T, DF, G>(sh, U, c.g, t, val, c.a, *c.ctr, c.df),
+              nacc_slots + (size_t)(*slot) * tab.nchains_total + c.index);
+}
+
+// One launch of either kind.
+struct GroupLaunch {
+  // one lattice
+  void *links = nullptr;
+  const Geom *g = nullptr;
+  const MetroArgs *a = nullptr;
+  const Defect *df = nullptr;
+  const uint32_t *d_sweep = nullptr;
+  // many chains
+  const ChainTable *tab = nullptr;
+  int blocks = 0;
+  const uint32_t *slot = nullptr;
+  int val = 0;
+  unsigned long long *nacc = nullptr;
+  cudaStream_t st = nullptr;
+};
+
+template <int NC, int ND, typename T, bool DF, int G> static cudaError_t launch_group_t(const GroupLaunch &l) {
+  if (l.tab) {
+    multi_group_kernel<NC, ND, T, DF, G><<<l.blocks, GROUP_THREADS, 0, l.st>>>(*l.tab, l.val, l.nacc, l.slot);
+    return cudaGetLastError();
+  }
+  const Geom &g = *l.g;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)group_blocks(g.Vh, G));
+  cfg.blockDim = dim3(GROUP_THREADS);
+  cfg.stream = l.st;
+  // the passes of a sweep after its first start before the one before has ended
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = l.val > 0 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, metropolis_group_kernel<NC, ND, T, DF, G>, Links<NC, T>{(cx<T> *)l.links, g.V}, g,
+                            l.val, *l.a, l.d_sweep, l.nacc, *l.df);
+}
+
+template <int NC, int ND, typename T> static cudaError_t launch_group_nd(int G, bool defect, const GroupLaunch &l) {
+  constexpr int SMALL = NC == 3 ? 8 : 16;
+  if constexpr (SharedStaples<NC, T>::v) {
+    if (defect)
+      return G == 32 ? launch_group_t<NC, ND, T, true, 32>(l) : launch_group_t<NC, ND, T, true, SMALL>(l);
+  } else {
+    if (defect) return cudaErrorInvalidValue;  // group_lanes gives 1
+  }
+  return G == 32 ? launch_group_t<NC, ND, T, false, 32>(l) : launch_group_t<NC, ND, T, false, SMALL>(l);
+}
+
+template <int NC> static cudaError_t launch_group_nc(int nd, int dtype, int G, bool defect, const GroupLaunch &l) {
+  if (dtype == 0) {
+    if (nd == 2) return launch_group_nd<NC, 2, double>(G, defect, l);
+    if (nd == 3) return launch_group_nd<NC, 3, double>(G, defect, l);
+    return launch_group_nd<NC, 4, double>(G, defect, l);
+  }
+  if (nd == 2) return launch_group_nd<NC, 2, float>(G, defect, l);
+  if (nd == 3) return launch_group_nd<NC, 3, float>(G, defect, l);
+  return launch_group_nd<NC, 4, float>(G, defect, l);
+}
+
+// per group, each in its own translation unit
+cudaError_t launch_group_u1(int nd, int dtype, int G, bool defect, const GroupLaunch &l);
+cudaError_t launch_group_su2(int nd, int dtype, int G, bool defect, const GroupLaunch &l);
+cudaError_t launch_group_su3(int nd, int dtype, int G, bool defect, const GroupLaunch &l);
+
+}  // namespace klft

@@ -137,6 +137,7 @@ template <int NC> struct HitDraws {
       return r;
     }
   }
+  template <typename T> KLFT_D bool accept(T dS, double u) const { return accept_uniform(dS, u); }
   // after the hit: drawn = the accept uniform was read
   KLFT_D void advance(bool drawn) {
     pos += used + (drawn ? 1u : 0u);
@@ -161,9 +162,9 @@ template <int NC> struct HitDraws {
 // The hits of link U_mu(x) in the reference's order (Metropolis.hpp:85-107),
 // drawing from the site's stream.  MU >= 0: mu at compile time (the staple's
 // site steps compiled, its nu loops unrolled); MU = -1: run-time mu.
-template <int NC, int ND, typename T, bool DF, int MU>
+template <int NC, int ND, typename T, bool DF, int MU, typename Draws>
 KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, int mu, const MetroArgs &a,
-                           const Defect &df, HitDraws<NC> &rng, long long lx, T bnc) {
+                           const Defect &df, Draws &rng, long long lx, T bnc) {
   if (open_link(g, x, mu)) return 0;
   int nacc = 0;
   Mat<NC, T> S;
@@ -191,7 +192,7 @@ KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
       T dS = -bnc * (tY - trO);
       if (dlink) dS *= (T)defect_c(df);
       const bool down = dS < T(0);
-      const bool accept = down || accept_uniform(dS, u);
+      const bool accept = down || rng.accept(dS, u);
       rng.advance(!down);
       if (accept) {
         A = Y;
@@ -214,7 +215,7 @@ KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
     T dS = -bnc * (retr_mul(rr, M) - trO);
     if (dlink) dS *= (T)defect_c(df);
     const bool down = dS < T(0);
-    const bool accept = down || accept_uniform(dS, u);
+    const bool accept = down || rng.accept(dS, u);
     rng.advance(!down);
     if (accept) {
       Uo = restore(mul(Uo, rr));
@@ -228,11 +229,11 @@ KLFT_D int link_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
   return nacc;
 }
 
-template <int NC, int ND, typename T, bool DF>
-KLFT_D int site_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, const MetroArgs &a, uint32_t sweep,
-                           const Defect &df) {
+// the links of a site in the order mu = 0 .. Nd-1, on the site's stream rng
+template <int NC, int ND, typename T, bool DF, typename Draws>
+KLFT_D int site_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, const MetroArgs &a, const Defect &df,
+                           Draws &rng) {
   int nacc = 0;
-  HitDraws<NC> rng(SiteStream(a.seed, a.chain, site_lex(g, x), sweep, KIND_METROPOLIS));
   const long long lx = site_lin(g, x);
   const T bnc = (T)a.beta / (T)NC;
   if constexpr (NC <= 2 && !DF) {
@@ -246,6 +247,13 @@ KLFT_D int site_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, 
     for (int mu = 0; mu < ND; ++mu) nacc += link_update_ref<NC, ND, T, DF, -1>(U, g, x, mu, a, df, rng, lx, bnc);
   }
   return nacc;
+}
+
+template <int NC, int ND, typename T, bool DF>
+KLFT_D int site_update_ref(const Links<NC, T> &U, const Geom &g, const Site &x, const MetroArgs &a, uint32_t sweep,
+                           const Defect &df) {
+  HitDraws<NC> rng(SiteStream(a.seed, a.chain, site_lex(g, x), sweep, KIND_METROPOLIS));
+  return site_update_ref<NC, ND, T, DF>(U, g, x, a, df, rng);
 }
 
 // SU(3) exp(i eps H) proposals U' = X U at fixed stream positions.  The

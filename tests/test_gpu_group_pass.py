@@ -1,0 +1,53 @@
+"""Reference-proposal passes by groups of lanes (small lattices): the same chain as
+the oracle's and as the pass with one thread per site, which a batch takes when
+its other chains make the launch large."""
+import numpy as np
+import pytest
+
+from klft_b200 import Batch, GaugeField
+
+pytestmark = pytest.mark.gpu
+
+BETA = {1: 1.0, 2: 2.3, 3: 5.7}
+DELTA = {1: 0.1, 2: 0.3, 3: 0.1}
+
+
+# sites per pass: a single one, ragged CTAs, either side of the changes of width
+# (800 and 2048); hits: none, one, more than a window of the stream holds
+@pytest.mark.parametrize("nc,L,nhits", [(1, [2, 2], 3), (1, [6, 4], 1), (1, [4, 6, 10], 70), (1, [14, 16, 16, 16], 2),
+                                        (2, [2, 2, 2], 5), (2, [4, 6, 8], 47), (2, [4, 4, 4, 6], 0),
+                                        (2, [14, 16, 16, 16], 3), (3, [2, 4], 9), (3, [8, 6, 10, 4], 33),
+                                        (3, [10, 12, 12, 12], 11)])
+def test_group_pass_follows_oracle(oracle, nc, L, nhits):
+    from oracle.oracle import Lat
+    lat = Lat(nc, L)
+    U = oracle.init(lat, True, 77)
+    g = GaugeField(L, nc, "fp64", "hot", 77)
+    g.set_stream(19, 3)
+    acc = g.metropolis(BETA[nc], DELTA[nc], nhits, 2)
+    acc_o = oracle.metropolis(lat, U, BETA[nc], DELTA[nc], nhits, 2, 19, chain=3)
+    np.testing.assert_array_equal(acc, np.nan_to_num(acc_o))  # no hits: the oracle's 0 / 0 is 0 here
+    np.testing.assert_allclose(g.download(), U, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("nc", [1, 2, 3])
+@pytest.mark.parametrize("precision,atol", [("fp64", 1e-12), ("mixed", 0.0)])
+@pytest.mark.parametrize("L,defect", [([8, 6, 4, 10], 0), ([8, 6, 4, 10], 2), ([12, 10, 6], 0), ([20, 14], 0)])
+def test_group_pass_is_the_chain_of_the_site_pass(nc, precision, atol, L, defect):
+    big = [24, 24, 24, 32] if len(L) == 4 else ([64, 56, 56] if len(L) == 3 else [320, 320])
+
+    def field(ext, seed):
+        g = GaugeField(ext, nc, precision, "hot", seed)
+        g.set_stream(seed, 1)
+        if defect:
+            g.set_defect(defect, (0, 1, 0), 0.5)
+        return g
+
+    alone, member, other = field(L, 5), field(L, 5), field(big, 6)
+    b = Batch()
+    for g in (member, other):
+        b.add(g, BETA[nc], DELTA[nc], 10)
+    acc, _, _, _ = b.run(3, False, False)
+    np.testing.assert_array_equal(alone.metropolis(BETA[nc], DELTA[nc], 10, 3), acc[:, 0])
+    np.testing.assert_allclose(alone.download(), member.download(), rtol=0, atol=atol)
+    b.close()
