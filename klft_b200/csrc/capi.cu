@@ -443,8 +443,7 @@ klft_status klft_staple_field(klft_lattice *lat, double *out) {
   const size_t bytes = (size_t)lat->g.V * lat->g.nd * lat->nc * lat->nc * 16;
   CK(lat->s_stage.ensure(bytes));
   CK(launch_staple_field(lat->nc, lat->dtype(), lat->links, lat->g, (double *)lat->s_stage.ptr, lat->stream));
-  CK(cudaMemcpyAsync(out, lat->s_stage.ptr, bytes, cudaMemcpyDeviceToHost, lat->stream));
-  CK(cudaStreamSynchronize(lat->stream));
+  CK(copy_result_to_host(out, lat->s_stage.ptr, bytes, lat->stream));
   return KLFT_OK;
 }
 

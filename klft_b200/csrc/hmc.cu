@@ -391,7 +391,7 @@ klft_status klft_hmc_set_momenta(klft_lattice *lat, const double *host) {
   if (s != KLFT_OK) return s;
   const size_t n = (size_t)lat->g.V * lat->g.nd * ncomp_of(lat->nc);
   CK(lat->s_stage.ensure(n * sizeof(double)));
-  CK(cudaMemcpyAsync(lat->s_stage.ptr, host, n * sizeof(double), cudaMemcpyHostToDevice, lat->stream));
+  CK(copy_host_to_device(lat->s_stage.ptr, host, n * sizeof(double), lat->stream));
   const unsigned grid = grid_for(lat->g.V * lat->g.nd, 256);
   if (lat->dtype() == 0)
     p_import_kernel<double><<<grid, 256, 0, lat->stream>>>((double *)b.P, lat->g, ncomp_of(lat->nc),
@@ -420,8 +420,7 @@ klft_status klft_hmc_get_momenta(klft_lattice *lat, double *host) {
     p_export_kernel<float><<<grid, 256, 0, lat->stream>>>((const float *)b.P, lat->g, ncomp_of(lat->nc),
                                                             (double *)lat->s_stage.ptr);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(host, lat->s_stage.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
-  CK(cudaStreamSynchronize(lat->stream));
+  CK(copy_result_to_host(host, lat->s_stage.ptr, n * sizeof(double), lat->stream));
   return KLFT_OK;
 }
 
@@ -455,8 +454,7 @@ klft_status klft_gauge_force(klft_lattice *lat, double beta, double *host_force)
     p_export_kernel<float><<<grid, 256, 0, lat->stream>>>((const float *)b.P, lat->g, ncomp_of(lat->nc),
                                                             (double *)lat->s_stage.ptr);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(host_force, lat->s_stage.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
-  CK(cudaStreamSynchronize(lat->stream));
+  CK(copy_result_to_host(host_force, lat->s_stage.ptr, n * sizeof(double), lat->stream));
   return KLFT_OK;
 }
 
