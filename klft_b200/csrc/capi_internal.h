@@ -42,6 +42,9 @@ cudaError_t copy_device_to_host(void *dst, const void *src, size_t bytes, cudaSt
 // are touched here for the first time, which many threads do no faster than the
 // driver's own copy below 32 MB (SU(3) 24^4 momenta, 85 MB: 19.4 -> 4.6 ms).
 cudaError_t copy_result_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
+// Momenta from the host, by the same paths: below 32 MB the driver's copy out of a
+// fresh array is 2 ms slower when its copy in was not the driver's.
+cudaError_t copy_input_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st);
 // Mixed form: only the stored FP32 reals of each link cross PCIe (12 for SU(3),
 // 4 for SU(2), 2 for U(1)); the host side converts from / to klft's 2 N^2
 // doubles per link (lexicographic site, then direction) on the library's threads.

@@ -391,7 +391,7 @@ klft_status klft_hmc_set_momenta(klft_lattice *lat, const double *host) {
   if (s != KLFT_OK) return s;
   const size_t n = (size_t)lat->g.V * lat->g.nd * ncomp_of(lat->nc);
   CK(lat->s_stage.ensure(n * sizeof(double)));
-  CK(copy_host_to_device(lat->s_stage.ptr, host, n * sizeof(double), lat->stream));
+  CK(copy_input_to_device(lat->s_stage.ptr, host, n * sizeof(double), lat->stream));
   const unsigned grid = grid_for(lat->g.V * lat->g.nd, 256);
   if (lat->dtype() == 0)
     p_import_kernel<double><<<grid, 256, 0, lat->stream>>>((double *)b.P, lat->g, ncomp_of(lat->nc),

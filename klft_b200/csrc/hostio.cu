@@ -370,6 +370,11 @@ cudaError_t copy_result_to_host(void *dst, const void *src, size_t bytes, cudaSt
   return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
+cudaError_t copy_input_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+  if (bytes >= kChunk) return copy_host_to_device(dst, src, bytes, st);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+}
+
 cudaError_t copy_host_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
   if (is_pinned(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   cudaError_t e = cudaSuccess;
