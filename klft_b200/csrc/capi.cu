@@ -382,9 +382,12 @@ klft_status klft_metropolis_sweeps(klft_lattice *lat, double beta, double delta,
 klft_status klft_plaquette(klft_lattice *lat, double *out) {
   if (!lat || !out) return fail(KLFT_EINVAL, "klft_plaquette: null pointer");
   LOCK(lat);
-  klft_status s = enqueue_plaquette(lat, 0);
-  if (s != KLFT_OK) return s;
-  CK(cudaMemcpyAsync(lat->h_results, lat->s_out.ptr, sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
+  // the sum goes straight into the handle's page-locked slots: a copy behind the
+  // kernels takes as long as they do on a small lattice
+  const int nblk = plaquette_blocks(lat->g);
+  CK(lat->s_part.ensure((size_t)nblk * sizeof(double)));
+  CK(launch_plaquette(lat->nc, lat->dtype(), lat->links, lat->g, (double *)lat->s_part.ptr, nblk, lat->h_results,
+                      lat->stream));
   CK(cudaStreamSynchronize(lat->stream));
   *out = normalize_plaquette(lat, lat->h_results[0]);
   return KLFT_OK;
@@ -421,11 +424,15 @@ klft_status klft_wilson_loop_temporal(klft_lattice *lat, const int *pairs, int n
   WilsonPlan plan;
   klft_status s = make_wilson_plan(lat, pairs, npairs, nd - 1, plan, 0, nd - 1);
   if (s != KLFT_OK) return s;
-  s = enqueue_wilson_spatial(lat, plan, false, (double *)lat->s_out.ptr, npairs);
+  // into the handle's page-locked slots when the sums fit (klft_plaquette)
+  const bool direct = nsum <= KLFT_RESULT_SLOTS;
+  s = enqueue_wilson_spatial(lat, plan, false, direct ? lat->h_results : (double *)lat->s_out.ptr, npairs);
   if (s != KLFT_OK) return s;
-  std::vector<double> sums(nsum);
-  CK(cudaMemcpyAsync(sums.data(), lat->s_out.ptr, nsum * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
+  std::vector<double> big(direct ? 0 : nsum);
+  if (!direct)
+    CK(cudaMemcpyAsync(big.data(), lat->s_out.ptr, nsum * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
   CK(cudaStreamSynchronize(lat->stream));
+  const double *sums = direct ? lat->h_results : big.data();
   for (int k = 0; k < npairs; ++k) {
     double acc = 0.0;
     for (int mu = 0; mu < nd - 1; ++mu) {
@@ -913,10 +920,13 @@ klft_status wilson_sums(klft_lattice *lat, int mu, int nu, const int *pairs, int
   WilsonPlan plan;
   klft_status s = make_wilson_plan(lat, pairs, npairs, nu, plan);
   if (s != KLFT_OK) return s;
-  s = enqueue_wilson_plane(lat, plan, mu, nu, false, (double *)lat->s_out.ptr);
+  const bool direct = npairs <= KLFT_RESULT_SLOTS;  // into the page-locked slots (klft_plaquette)
+  s = enqueue_wilson_plane(lat, plan, mu, nu, false, direct ? lat->h_results : (double *)lat->s_out.ptr);
   if (s != KLFT_OK) return s;
-  CK(cudaMemcpyAsync(sums, lat->s_out.ptr, (size_t)npairs * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
+  if (!direct)
+    CK(cudaMemcpyAsync(sums, lat->s_out.ptr, (size_t)npairs * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
   CK(cudaStreamSynchronize(lat->stream));
+  if (direct) std::memcpy(sums, lat->h_results, (size_t)npairs * sizeof(double));
   return KLFT_OK;
 }
 

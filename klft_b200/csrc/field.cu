@@ -3,6 +3,7 @@
 // reunitarisation, the unitarity monitor and the all-links staple field.
 #include "group.cuh"
 #include "kernels.cuh"
+#include "pdl.cuh"
 #include "staple.cuh"
 
 namespace klft {
@@ -93,6 +94,8 @@ __global__ void export_f32_kernel(Links<NC, float> U, Geom g, float *__restrict_
 template <int NC, typename T>
 __global__ void reunitarize_kernel(Links<NC, T> U, Geom g) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (t >= g.V * g.nd) return;
   const int mu = (int)(t / g.V);
   const long long lin = t - (long long)mu * g.V;
@@ -243,10 +246,11 @@ cudaError_t launch_export(int nc, int dtype, const void *links, const Geom &g, d
   return cudaGetLastError();
 }
 
-cudaError_t launch_reunitarize(int nc, int dtype, void *links, const Geom &g, cudaStream_t st) {
-  KLFT_DISPATCH_NC_T(nc, dtype, (reunitarize_kernel<NC, T><<<nblocks(g.V * g.nd, 256), 256, 0, st>>>(
-                                    Links<NC, T>{(cx<T> *)links, g.V}, g)));
-  return cudaGetLastError();
+cudaError_t launch_reunitarize(int nc, int dtype, void *links, const Geom &g, cudaStream_t st, bool dependent) {
+  cudaError_t e = cudaSuccess;
+  KLFT_DISPATCH_NC_T(nc, dtype, (e = launch_after(dependent, reunitarize_kernel<NC, T>, dim3(nblocks(g.V * g.nd, 256)),
+                                                  dim3(256), 0, st, Links<NC, T>{(cx<T> *)links, g.V}, g)));
+  return e;
 }
 
 cudaError_t launch_open_boundary(int nc, int dtype, void *links, const Geom &g, cudaStream_t st) {

@@ -19,6 +19,7 @@
 #include "capi_internal.h"
 #include "group.cuh"
 #include "kernels.cuh"
+#include "pdl.cuh"
 #include "staple.cuh"
 
 namespace klft {
@@ -34,6 +35,8 @@ __global__ void __launch_bounds__(HMC_THREADS) momenta_kernel(T *P, Geom g, uint
   const long long lin = t - (long long)mu * g.V;
   const Site x = site_from_lin(g, lin);
   constexpr int nc = Alg<NC>::n;
+  grid_dependency_wait();
+  grid_launch_dependents();
   Stream st(seed, chain, site_lex(g, x), ctr[1], KIND_MOMENTUM, (uint32_t)mu);
   double gs[8];
 #pragma unroll
@@ -52,6 +55,8 @@ __global__ void __launch_bounds__(128) force_update_kernel(Links<NC, T> U, T *P,
   if (lin >= g.V) return;
   const int mu = (int)blockIdx.y;
   const Site x = g.Vh < (1LL << 31) ? site_from_lin32(g, (unsigned)lin) : site_from_lin(g, lin);
+  grid_dependency_wait();
+  grid_launch_dependents();
   Mat<NC, T> S;
   if constexpr (NC == 3) {
     // SU(3): the rolled staple (the unrolled products cost occupancy: 150 registers)
@@ -79,6 +84,8 @@ __global__ void __launch_bounds__(HMC_THREADS) gauge_update_kernel(Links<NC, T> 
   const int mu = (int)(t / g.V);
   const long long lin = t - (long long)mu * g.V;
   constexpr int nc = Alg<NC>::n;
+  grid_dependency_wait();
+  grid_launch_dependents();
   T p[nc];
 #pragma unroll
   for (int a = 0; a < nc; ++a) p[a] = P[((long long)mu * nc + a) * g.V + lin];
@@ -88,6 +95,8 @@ __global__ void __launch_bounds__(HMC_THREADS) gauge_update_kernel(Links<NC, T> 
 // sum of p^2 / 2 over the field, FP64, block partials
 template <typename T>
 __global__ void __launch_bounds__(HMC_THREADS) kinetic_kernel(const T *P, long long n, double *part) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   double acc = 0.0;
   for (long long i = (long long)blockIdx.x * HMC_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * HMC_THREADS) {
     const double p = (double)P[i];
@@ -110,6 +119,8 @@ __global__ void __launch_bounds__(HMC_THREADS) kinetic_kernel(const T *P, long l
 // counter.
 __global__ void hmc_accept_kernel(const double *slots, double bnc, uint64_t seed, uint64_t chain, uint32_t *ctr,
                                   double *dH_out, int *acc_out) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const double g_old = -bnc * slots[1], g_new = -bnc * slots[3];
   double dH = 0.0;
   dH += slots[2] - slots[0];
@@ -126,6 +137,8 @@ __global__ void hmc_accept_kernel(const double *slots, double bnc, uint64_t seed
 
 // restore the saved links of a rejected trajectory
 __global__ void restore_if_rejected_kernel(uint4 *links, const uint4 *saved, long long n16, const int *accepted) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (*accepted) return;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (long long)gridDim.x * blockDim.x)
     links[i] = saved[i];
@@ -151,43 +164,52 @@ static unsigned grid_for(long long n, int b) { return (unsigned)((n + b - 1) / b
 
 static int ncomp_of(int nc) { return nc == 1 ? 1 : (nc == 2 ? 3 : 8); }
 
-cudaError_t launch_momenta(const klft_lattice *lat, void *P) {
+// dependent (here and below): the operation before in the stream is a kernel (pdl.cuh)
+cudaError_t launch_momenta(const klft_lattice *lat, void *P, bool dependent = false) {
   const Geom &g = lat->g;
+  cudaError_t e = cudaSuccess;
   KLFT_HMC_DISPATCH(lat->nc, lat->dtype(),
-                    (momenta_kernel<NC, T><<<grid_for(g.V * g.nd, HMC_THREADS), HMC_THREADS, 0, lat->stream>>>(
-                        (T *)P, g, lat->seed, lat->chain, lat->d_counters)));
-  return cudaGetLastError();
+                    (e = launch_after(dependent, momenta_kernel<NC, T>, dim3(grid_for(g.V * g.nd, HMC_THREADS)),
+                                      dim3(HMC_THREADS), 0, lat->stream, (T *)P, g, lat->seed, lat->chain,
+                                      (const uint32_t *)lat->d_counters)));
+  return e;
 }
 
-cudaError_t launch_force_update(const klft_lattice *lat, void *P, double beta, double dt) {
+cudaError_t launch_force_update(const klft_lattice *lat, void *P, double beta, double dt, bool dependent = false) {
   const Geom &g = lat->g;
+  cudaError_t e = cudaSuccess;
 #define KLFT_FU(NDV)                                                                                        \
-  force_update_kernel<NC, NDV, T><<<dim3(grid_for(g.V, 128), NDV), 128, 0, lat->stream>>>(                   \
-      Links<NC, T>{(cx<T> *)lat->links, g.V}, (T *)P, g, (T)(beta / (double)NC), (T)dt)
+  e = launch_after(dependent, force_update_kernel<NC, NDV, T>, dim3(grid_for(g.V, 128), NDV), dim3(128), 0,    \
+                   lat->stream, Links<NC, T>{(cx<T> *)lat->links, g.V}, (T *)P, g, (T)(beta / (double)NC), (T)dt)
   KLFT_HMC_DISPATCH(lat->nc, lat->dtype(), ({
     if (g.nd == 2) KLFT_FU(2);
     else if (g.nd == 3) KLFT_FU(3);
     else KLFT_FU(4);
   }));
 #undef KLFT_FU
-  return cudaGetLastError();
+  return e;
 }
 
-cudaError_t launch_gauge_update(const klft_lattice *lat, const void *P, double dt) {
+cudaError_t launch_gauge_update(const klft_lattice *lat, const void *P, double dt, bool dependent = false) {
   const Geom &g = lat->g;
+  cudaError_t e = cudaSuccess;
   KLFT_HMC_DISPATCH(lat->nc, lat->dtype(),
-                    (gauge_update_kernel<NC, T><<<grid_for(g.V * g.nd, HMC_THREADS), HMC_THREADS, 0, lat->stream>>>(
-                        Links<NC, T>{(cx<T> *)lat->links, g.V}, (const T *)P, g, (T)dt)));
-  return cudaGetLastError();
+                    (e = launch_after(dependent, gauge_update_kernel<NC, T>, dim3(grid_for(g.V * g.nd, HMC_THREADS)),
+                                      dim3(HMC_THREADS), 0, lat->stream, Links<NC, T>{(cx<T> *)lat->links, g.V},
+                                      (const T *)P, g, (T)dt)));
+  return e;
 }
 
-cudaError_t launch_kinetic(const klft_lattice *lat, const void *P, double *d_part, int nblk, double *d_out) {
+cudaError_t launch_kinetic(const klft_lattice *lat, const void *P, double *d_part, int nblk, double *d_out,
+                           bool dependent = false) {
   const long long n = lat->g.V * lat->g.nd * ncomp_of(lat->nc);
+  cudaError_t e;
   if (lat->dtype() == 0)
-    kinetic_kernel<double><<<nblk, HMC_THREADS, 0, lat->stream>>>((const double *)P, n, d_part);
+    e = launch_after(dependent, kinetic_kernel<double>, dim3(nblk), dim3(HMC_THREADS), 0, lat->stream, (const double *)P,
+                     n, d_part);
   else
-    kinetic_kernel<float><<<nblk, HMC_THREADS, 0, lat->stream>>>((const float *)P, n, d_part);
-  cudaError_t e = cudaGetLastError();
+    e = launch_after(dependent, kinetic_kernel<float>, dim3(nblk), dim3(HMC_THREADS), 0, lat->stream, (const float *)P,
+                     n, d_part);
   if (e != cudaSuccess) return e;
   return launch_reduce_partials(d_part, nblk, 1, d_out, lat->stream);
 }
@@ -238,11 +260,12 @@ klft_status hmc_bufs(klft_lattice *lat, int ntraj, HmcBufs &b) {
   return KLFT_OK;
 }
 
-klft_status enqueue_energies(klft_lattice *lat, const HmcBufs &b, double *slot_k, double *slot_p) {
+klft_status enqueue_energies(klft_lattice *lat, const HmcBufs &b, double *slot_k, double *slot_p,
+                             bool dependent = false) {
   const int nblk = plaquette_blocks(lat->g);
-  CK(launch_kinetic(lat, b.P, (double *)lat->s_part.ptr, nblk, slot_k));
+  CK(launch_kinetic(lat, b.P, (double *)lat->s_part.ptr, nblk, slot_k, dependent));
   CK(launch_plaquette(lat->nc, lat->dtype(), lat->links, lat->g, (double *)lat->s_part.ptr, nblk, slot_p,
-                      lat->stream, -1, true));
+                      lat->stream, -1, true, true));
   return KLFT_OK;
 }
 
@@ -254,12 +277,15 @@ klft_status enqueue_energies(klft_lattice *lat, const HmcBufs &b, double *slot_k
 klft_status enqueue_integrate(klft_lattice *lat, const HmcBufs &b, double beta, double tau, int nsteps,
                               int integrator) {
   const double dt = (lat->hmc_generators == KLFT_GENERATORS_HALF ? 0.5 : 1.0) * tau / (double)nsteps;
+  bool dependent = false;  // after the first kernel
   auto P = [&](double h) -> klft_status {
-    CK(launch_force_update(lat, b.P, beta, h));
+    CK(launch_force_update(lat, b.P, beta, h, dependent));
+    dependent = true;
     return KLFT_OK;
   };
   auto U = [&](double h) -> klft_status {
-    CK(launch_gauge_update(lat, b.P, h));
+    CK(launch_gauge_update(lat, b.P, h, dependent));
+    dependent = true;
     return KLFT_OK;
   };
   klft_status s = KLFT_OK;
@@ -290,7 +316,7 @@ klft_status enqueue_integrate(klft_lattice *lat, const HmcBufs &b, double beta, 
     }
   }
 #undef STEP
-  CK(launch_reunitarize(lat->nc, lat->dtype(), lat->links, lat->g, lat->stream));
+  CK(launch_reunitarize(lat->nc, lat->dtype(), lat->links, lat->g, lat->stream, dependent));
   return KLFT_OK;
 }
 
@@ -357,16 +383,14 @@ klft_status hmc_enqueue_trajectory(klft_lattice *lat, double beta, double tau, i
   klft_status s = hmc_bufs(lat, k + 1, b);
   if (s != KLFT_OK) return s;
   CK(launch_momenta(lat, b.P));
-  if ((s = enqueue_energies(lat, b, b.slots + 0, b.slots + 1)) != KLFT_OK) return s;
+  if ((s = enqueue_energies(lat, b, b.slots + 0, b.slots + 1, true)) != KLFT_OK) return s;
   CK(cudaMemcpyAsync(b.saved, lat->links, lat->link_bytes, cudaMemcpyDeviceToDevice, lat->stream));
   if ((s = enqueue_integrate(lat, b, beta, tau, nsteps, integrator)) != KLFT_OK) return s;
-  if ((s = enqueue_energies(lat, b, b.slots + 2, b.slots + 3)) != KLFT_OK) return s;
-  hmc_accept_kernel<<<1, 1, 0, lat->stream>>>(b.slots, beta / (double)lat->nc, lat->seed, lat->chain,
-                                              lat->d_counters, b.dH + k, b.acc + k);
-  CK(cudaGetLastError());
-  restore_if_rejected_kernel<<<296, 256, 0, lat->stream>>>((uint4 *)lat->links, (const uint4 *)b.saved,
-                                                           (long long)(lat->link_bytes / 16), b.acc + k);
-  CK(cudaGetLastError());
+  if ((s = enqueue_energies(lat, b, b.slots + 2, b.slots + 3, true)) != KLFT_OK) return s;
+  CK(launch_after(true, hmc_accept_kernel, dim3(1), dim3(1), 0, lat->stream, (const double *)b.slots,
+                  beta / (double)lat->nc, lat->seed, lat->chain, lat->d_counters, b.dH + k, b.acc + k));
+  CK(launch_after(true, restore_if_rejected_kernel, dim3(296), dim3(256), 0, lat->stream, (uint4 *)lat->links,
+                  (const uint4 *)b.saved, (long long)(lat->link_bytes / 16), (const int *)(b.acc + k)));
   return KLFT_OK;
 }
 

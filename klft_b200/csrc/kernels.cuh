@@ -45,7 +45,7 @@ cudaError_t launch_import_f32(int nc, void *links, const Geom &g, const float *a
 cudaError_t launch_export_f32(int nc, const void *links, const Geom &g, float *aos, cudaStream_t st);
 // zero the links across the open boundary (no-op when periodic)
 cudaError_t launch_open_boundary(int nc, int dtype, void *links, const Geom &g, cudaStream_t st);
-cudaError_t launch_reunitarize(int nc, int dtype, void *links, const Geom &g, cudaStream_t st);
+cudaError_t launch_reunitarize(int nc, int dtype, void *links, const Geom &g, cudaStream_t st, bool dependent = false);
 // max ||U^dagger U - 1||_F -> *d_out (via partials)
 cudaError_t launch_unitarity(int nc, int dtype, const void *links, const Geom &g, double *d_part, double *d_out,
                              cudaStream_t st);
@@ -54,8 +54,10 @@ cudaError_t launch_staple_field(int nc, int dtype, const void *links, const Geom
 
 // sum over sites of sum_{mu<nu<nu_end} Re Tr P_{mu nu} (nu_end < 0: all planes), unnormalised, into *d_out;
 // f64_terms: every product term summed in FP64 (else each plane's trace in the link precision)
+// dependent: the operation before in st is a kernel (pdl.cuh)
 cudaError_t launch_plaquette(int nc, int dtype, const void *links, const Geom &g, double *d_part, int nblk,
-                             double *d_out, cudaStream_t st, int nu_end = -1, bool f64_terms = false);
+                             double *d_out, cudaStream_t st, int nu_end = -1, bool f64_terms = false,
+                             bool dependent = false);
 // Wilson loops of a pair list in the (mu, nu) plane; d_out[k] = sum over sites Re Tr W
 cudaError_t launch_wilson_direct(int nc, int dtype, const void *links, const Geom &g, int mu, int nu,
                                  const int *d_pairs, int npairs, double *d_part, int nblk, double *d_out,

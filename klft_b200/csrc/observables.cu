@@ -13,12 +13,15 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "observables.cuh"
+#include "pdl.cuh"
 
 namespace klft {
 
 template <int NC, int ND, typename T, bool F64>
 __global__ void __launch_bounds__(RED_THREADS, PlaqMinBlocks<T>::v) plaquette_kernel(Links<NC, T> U, Geom g,
                                                                                      double *part, int nu_end) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const double s =
       block_sum<RED_THREADS>(plaquette_partial<NC, ND, T, F64>(U, g, nu_end, blockIdx.x, gridDim.x));
   if (threadIdx.x == 0) part[blockIdx.x] = s;
@@ -67,6 +70,8 @@ __global__ void __launch_bounds__(RED_THREADS) wilson_direct_kernel(Links<NC, T>
 // out[k] = sum_i part[k * nblk + i], one block per output, fixed order
 __global__ void reduce_partials_kernel(const double *part, int nblk, double *out) {
   const int k = blockIdx.x;
+  grid_dependency_wait();
+  grid_launch_dependents();
   double v = 0.0;
   for (int i = threadIdx.x; i < nblk; i += RED_THREADS) v += part[(long long)k * nblk + i];
   const double s = block_sum<RED_THREADS>(v);
@@ -80,8 +85,8 @@ int plaquette_blocks(const Geom &g) {
 
 cudaError_t launch_reduce_partials(const double *d_part, int nblk, int n, double *d_out, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  reduce_partials_kernel<<<n, RED_THREADS, 0, st>>>(d_part, nblk, d_out);
-  return cudaGetLastError();
+  // always right behind the kernel that wrote the partials
+  return launch_after(true, reduce_partials_kernel, dim3(n), dim3(RED_THREADS), 0, st, d_part, nblk, d_out);
 }
 
 #define KLFT_OBS_DISPATCH(nc, dtype, nd, KERNEL_CALL)                           \
@@ -102,16 +107,14 @@ cudaError_t launch_reduce_partials(const double *d_part, int nblk, int n, double
   } while (0)
 
 cudaError_t launch_plaquette(int nc, int dtype, const void *links, const Geom &g, double *d_part, int nblk,
-                             double *d_out, cudaStream_t st, int nu_end, bool f64_terms) {
+                             double *d_out, cudaStream_t st, int nu_end, bool f64_terms, bool dependent) {
   if (nu_end < 0) nu_end = g.nd;
+  cudaError_t e = cudaSuccess;
 #define KLFT_PQ(NDV)                                                                                              \
   do {                                                                                                            \
-    if (f64_terms)                                                                                                \
-      plaquette_kernel<NC, NDV, T, true><<<nblk, RED_THREADS, 0, st>>>(Links<NC, T>{(cx<T> *)links, g.V}, g,      \
-                                                                       d_part, nu_end);                           \
-    else                                                                                                          \
-      plaquette_kernel<NC, NDV, T, false><<<nblk, RED_THREADS, 0, st>>>(Links<NC, T>{(cx<T> *)links, g.V}, g,     \
-                                                                        d_part, nu_end);                          \
+    const Links<NC, T> U{(cx<T> *)links, g.V};                                                                    \
+    e = launch_after(dependent, f64_terms ? plaquette_kernel<NC, NDV, T, true> : plaquette_kernel<NC, NDV, T, false>, \
+                     dim3(nblk), dim3(RED_THREADS), 0, st, U, g, d_part, nu_end);                                  \
   } while (0)
   KLFT_OBS_DISPATCH(nc, dtype, g.nd, ({
     if (g.nd == 2) KLFT_PQ(2);
@@ -119,7 +122,6 @@ cudaError_t launch_plaquette(int nc, int dtype, const void *links, const Geom &g
     else KLFT_PQ(4);
   }));
 #undef KLFT_PQ
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_reduce_partials(d_part, nblk, 1, d_out, st);
 }

@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "pdl.cuh"
 
 namespace klft {
 
@@ -227,6 +228,8 @@ __global__ void __launch_bounds__(32 * UP_RB) uprime_kernel(Links<N, T> U, Geom 
   const long long col = ctile * 32 + cl;
   const int row = row0 + r;
   const int Ln = c.Lnu;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (col < c.ncols && row < c.rows) {
     const int b = row % Ln, k = row / Ln;
     int x[4];
@@ -409,6 +412,8 @@ __global__ void __launch_bounds__(WL_THREADS, WLMinBlocks<T>::v)
   unsigned char *S = smem_raw + (((size_t)w.npairs * WL_WARPS * sizeof(double) + 15) & ~(size_t)15);  // entries
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int p = tid; p < w.npairs * WL_WARPS; p += WL_THREADS) acc[p] = 0.0;
+  grid_dependency_wait();
+  grid_launch_dependents();
   __syncthreads();
   const int Ln = c.Lnu;
   // columns never straddle a warp when QR divides 32: warp-level sync suffices
@@ -641,6 +646,8 @@ __global__ void __launch_bounds__(WC_THREADS, WCMinBlocks<T>::v)
   T *buf = (T *)smem_raw;                                   // [2][WC_CW][CS]
   double *acc = (double *)(buf + 2 * WC_CW * CS);          // [nplanes * npairs][WC_WARPS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int cc = tid / WC_PT, q = tid % WC_PT;
   for (int i = tid; i < 2 * WC_CW * CS; i += WC_THREADS) buf[i] = T(0);  // rows never written stay finite
   const int nout = w.nplanes * w.npairs;
@@ -816,8 +823,11 @@ static cudaError_t wilson_gf_t(const void *links, const Geom &g, const int *cons
   const long long nct = (c[0].ncols + 31) / 32;
   for (int i = 0; i < nplanes; ++i) {
     const CField<N, T> up{(cx<T> *)(up0 + i * up_bytes), c[i].ncols * c[i].rows};
-    uprime_kernel<N, T><<<(unsigned)(nct * ((c[i].rows + UP_RB - 1) / UP_RB)), 32 * UP_RB, 0, st>>>(U, g, c[i], om,
-                                                                                                 pol, up);
+    // behind Omega or the plane before
+    const cudaError_t e = launch_after(!omega_ready || i > 0, uprime_kernel<N, T>,
+                                       dim3((unsigned)(nct * ((c[i].rows + UP_RB - 1) / UP_RB))), dim3(32 * UP_RB), 0,
+                                       st, U, g, c[i], om, pol, up);
+    if (e != cudaSuccess) return e;
   }
   // the loop kernels read U' only: on stl (if given) after U' is complete
   if (stl) {
@@ -866,8 +876,8 @@ static cudaError_t wilson_gf_t(const void *links, const Geom &g, const int *cons
       }();
       const long long ntiles = w.ntiles1 * nplanes;
       const int grid = (int)std::min<long long>(std::min<long long>(want, nblk), ntiles > 0 ? ntiles : 1);
-      wcorr_kernel<N, T><<<grid, WC_THREADS, smem, st>>>(up, c[0], w, tmax, d_part);
-      cudaError_t e = cudaGetLastError();
+      const cudaError_t e = launch_after(!stl, wcorr_kernel<N, T>, dim3(grid), dim3(WC_THREADS), smem, st, up, c[0], w,
+                                         tmax, d_part);
       if (e != cudaSuccess) return e;
       *grid_used = grid;
       return cudaSuccess;
