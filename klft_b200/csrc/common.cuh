@@ -413,6 +413,18 @@ KLFT_HD Site site_dn(const Geom &g, Site s, int d) {
   }
   return s;
 }
+// lin(x + e_d) - lin(x) and lin(x - e_d) - lin(x) (volumes below 2^31).  A step in
+// one dimension changes lin by an amount that depends on that coordinate alone, so
+// the index of x + e_mu - e_nu is a sum of two steps: the kernels that read many
+// neighbours form each step once instead of a site and its index per neighbour.
+KLFT_HD int step_up(const Geom &g, const Site &s, int d) {
+  const int c = (int)g.Vh << d;
+  return s.b(d) == 0 ? c : (s.h(d) + 1 == g.Hd(d) ? -c - s.h(d) * g.hs[d] : g.hs[d] - c);
+}
+KLFT_HD int step_dn(const Geom &g, const Site &s, int d) {
+  const int c = (int)g.Vh << d;
+  return s.b(d) == 1 ? -c : (s.h(d) == 0 ? c + (g.Hd(d) - 1) * g.hs[d] : c - g.hs[d]);
+}
 // x + k e_d, any k >= 0 (periodic)
 KLFT_HD Site site_shift(const Geom &g, Site s, int d, int k) {
   int x = 2 * s.h(d) + s.b(d);

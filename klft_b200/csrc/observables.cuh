@@ -68,6 +68,7 @@ template <> struct PlaqMinBlocks<double> { static constexpr int v = 1; };
 // precision and the lattice sum in FP64.
 template <int NC, int ND, typename T, bool F64 = false>
 KLFT_D double plaquette_partial(const Links<NC, T> &U, const Geom &g, int nu_end, long long b, long long nb) {
+  constexpr bool steps = NC == 3 || sizeof(T) == 8;  // as in staple_ct
   double acc = 0.0;
   const long long nthr = window_threads(g);
   for (long long t = b * RED_THREADS + threadIdx.x; t < nthr; t += nb * RED_THREADS) {
@@ -82,8 +83,8 @@ KLFT_D double plaquette_partial(const Links<NC, T> &U, const Geom &g, int nu_end
 #pragma unroll
       for (int nu = mu + 1; nu < ND; ++nu) {
         if (nu >= nu_end) break;
-        const Mat<NC, T> lmu = mul(umu, U.load(site_lin(g, xpmu), nu));
-        const Mat<NC, T> lnu = mul(U.load(lin, nu), U.load(site_lin(g, site_up(g, x, nu)), mu));
+        const Mat<NC, T> lmu = mul(umu, U.load(steps ? lin + step_up(g, x, mu) : site_lin(g, xpmu), nu));
+        const Mat<NC, T> lnu = mul(U.load(lin, nu), U.load(steps ? lin + step_up(g, x, nu) : site_lin(g, site_up(g, x, nu)), mu));
         if constexpr (F64) acc += retr_nd<NC, T, double>(lmu, lnu);
         else acc += (double)retr_nd<NC, T, T>(lmu, lnu);
       }

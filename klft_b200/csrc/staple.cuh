@@ -86,27 +86,25 @@ template <typename T> KLFT_D void mul_dn_rows01(const Mat<3, T> &a, const Mat<3,
 template <int ND, int MU>
 KLFT_D Mat<3, float> staple_su3_2row_ct(const Links<3, float> &U, const Geom &g, const Site &x) {
   Mat<3, float> S = mzero<3, float>();
-  const Site xpmu = site_up(g, x, MU);
+  const int lin = (int)site_lin(g, x), pmu = lin + step_up(g, x, MU);
 #pragma unroll
   for (int nu = 0; nu < ND; ++nu) {
     if (nu == MU) continue;
-    const Site xpnu = site_up(g, x, nu);
     Mat<3, float> cb, f;
-    mul_rows01(U.load_rows01(site_lin(g, x), nu), U.load(site_lin(g, xpnu), MU), cb);
+    mul_rows01(U.load_rows01(lin, nu), U.load(lin + step_up(g, x, nu), MU), cb);
     complete_row2(cb);
-    mul_nd_rows01(U.load_rows01(site_lin(g, xpmu), nu), cb, f);
+    mul_nd_rows01(U.load_rows01(pmu, nu), cb, f);
     complete_row2(f);
     madd(S, f);
   }
 #pragma unroll
   for (int nu = 0; nu < ND; ++nu) {
     if (nu == MU) continue;
-    const Site xpmu_mnu = site_dn(g, xpmu, nu);
-    const Site xmnu = site_dn(g, x, nu);
+    const int dn = step_dn(g, x, nu);
     Mat<3, float> ed, f;
-    mul_rows01(U.load_rows01(site_lin(g, xmnu), MU), U.load(site_lin(g, xpmu_mnu), nu), ed);
+    mul_rows01(U.load_rows01(lin + dn, MU), U.load(pmu + dn, nu), ed);
     complete_row2(ed);
-    mul_dn_rows01(ed, U.load(site_lin(g, xmnu), nu), f);
+    mul_dn_rows01(ed, U.load(lin + dn, nu), f);
     complete_row2(f);
     madd(S, f);
   }
@@ -122,6 +120,26 @@ KLFT_D Mat<3, float> staple_su3_2row_ct(const Links<3, float> &U, const Geom &g,
 template <int NC, int ND, int MU, typename T, bool DF = false>
 KLFT_D Mat<NC, T> staple_ct(const Links<NC, T> &U, const Geom &g, const Site &x, const Defect &df = Defect{}) {
   Mat<NC, T> S = mzero<NC, T>();
+  if constexpr (!DF && (NC == 3 || sizeof(T) == 8)) {
+    // neighbours as sums of two steps.  Not in FP32 for U(1) and SU(2): the compiler
+    // contracts their sums of two products in another order then, and the chain's
+    // last bits (HMC's dH, Metropolis decisions) with them.
+    const int lin = (int)site_lin(g, x), pmu = lin + step_up(g, x, MU);
+#pragma unroll
+    for (int nu = 0; nu < ND; ++nu) {
+      if (nu == MU) continue;
+      const Mat<NC, T> t = mul_nd(U.load(pmu, nu), U.load(lin + step_up(g, x, nu), MU));
+      madd(S, mul_nd(t, U.load(lin, nu)));
+    }
+#pragma unroll
+    for (int nu = 0; nu < ND; ++nu) {
+      if (nu == MU) continue;
+      const int dn = step_dn(g, x, nu);
+      const Mat<NC, T> t = mul_dd(U.load(pmu + dn, nu), U.load(lin + dn, MU));
+      madd(S, mul(t, U.load(lin + dn, nu)));
+    }
+    return S;
+  }
   const Site xpmu = site_up(g, x, MU);
 #pragma unroll
   for (int nu = 0; nu < ND; ++nu) {
