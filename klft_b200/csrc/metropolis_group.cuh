@@ -27,11 +27,9 @@
 #pragma once
 #include "chains.cuh"
 #include "metropolis_site.cuh"
+#include "pdl.cuh"
 
 namespace klft {
-
-KLFT_D void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-KLFT_D void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <int G> KLFT_D unsigned group_mask() {
   if constexpr (G == 32) return 0xffffffffu;
@@ -61,7 +59,6 @@ template <int NC, typename T, int G> struct TableDraws {
   const unsigned mask;  // the group's lanes
   int wn = 0, i = 0;    // window: places [base, base + wn) of the stream; the next hit's place
   uint32_t base = 0;
-  bool have = false;
   cx<T> r[NC], ra[NC], rb[NC];  // row 0 of this hit's proposal, of the two that can come next
   float lg = 0.f, la = 0.f, lb = 0.f;
 
@@ -91,17 +88,20 @@ template <int NC, typename T, int G> struct TableDraws {
       for (int j = 0; j < NC; ++j) tab.prop[p][j] = m.e[0][j];
     }
     __syncwarp(mask);
-    have = false;
   }
 
-  template <typename> KLFT_D Mat<NC, T> propose_next(double, double &) {
+  // the number of hits, up to `hits` (>= 1), that the window surely holds
+  KLFT_D int ready(int hits) {
     if (i + K >= wn) fill();
-    if (!have) {
+    const int sure = (wn - i) / (K + 1);
+    const int m = hits < sure ? hits : (sure > 1 ? sure : 1);
+    left -= m;
 #pragma unroll
-      for (int j = 0; j < NC; ++j) r[j] = tab.prop[i][j];
-      lg = tab.lg[i + K];
-      have = true;
-    }
+    for (int j = 0; j < NC; ++j) r[j] = tab.prop[i][j];
+    lg = tab.lg[i + K];
+    return m;
+  }
+  KLFT_D Mat<NC, T> propose_next() {
     // both places the next hit can be at, loaded beside this hit's arithmetic
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
@@ -110,7 +110,6 @@ template <int NC, typename T, int G> struct TableDraws {
     }
     la = tab.lg[i + 2 * K];
     lb = tab.lg[i + 2 * K + 1];
-    --left;
     Mat<NC, T> m;
 #pragma unroll
     for (int j = 0; j < NC; ++j) m.e[0][j] = r[j];
@@ -119,10 +118,10 @@ template <int NC, typename T, int G> struct TableDraws {
   }
   // u < exp(-dS) from ln u <= 0 in FP32 (absolute error below 2e-5); within 1e-4, and
   // for u = 0 or a NaN, the accurate comparison of accept_uniform
-  KLFT_D bool accept(T dS, double) const {
+  KLFT_D bool accept(T dS) const {
     const float t = (float)dS + lg;
-    if (fabsf(t) > 1e-4f) return t < 0.f;
-    return tab.u[i + K] < (double)exp(-dS);
+    if (__builtin_expect(!(fabsf(t) > 1e-4f), 0)) return dS < T(0) || tab.u[i + K] < (double)exp(-dS);
+    return t < 0.f;
   }
   KLFT_D void advance(bool drawn) {
     i += drawn ? K + 1 : K;
@@ -165,18 +164,21 @@ KLFT_D int group_hits(const Mat<NC, T> &S, Mat<NC, T> &Uo, const MetroArgs &a, b
   T trO = retr_diag(M0);
   int nacc = 0;
 #pragma unroll 1
-  for (int hit = 0; hit < a.nhits; ++hit) {
-    double u;
-    const Mat<NC, T> Y = mul(A, rng.template propose_next<T>(a.delta, u));
-    const T tY = retr_mul(Y, M0);
-    const T dS = -bnc * (tY - trO) * cdef;
-    const bool down = dS < T(0);
-    const bool accept = down || rng.accept(dS, u);
-    rng.advance(!down);
-    if (accept) {
-      A = Y;
-      trO = tY;
-      ++nacc;
+  for (int hit = 0; hit < a.nhits;) {
+    const int m = rng.ready(a.nhits - hit);
+    hit += m;
+#pragma unroll 1
+    for (int k = 0; k < m; ++k) {
+      const Mat<NC, T> Y = mul(A, rng.propose_next());
+      const T tY = retr_mul(Y, M0);
+      const T dS = -bnc * (tY - trO) * cdef;
+      const bool accept = rng.accept(dS);  // ln u <= 0: also of dS < 0
+      rng.advance(!(dS < T(0)));
+      if (accept) {
+        A = Y;
+        trO = tY;
+        ++nacc;
+      }
     }
   }
   if (nacc) Uo = restore(mul(U0, A));
@@ -267,18 +269,21 @@ KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &
     float trO = group_retr(M0);
     int nacc = 0;
 #pragma unroll 1
-    for (int hit = 0; hit < a.nhits; ++hit) {
-      double u;
-      const Row0<NC> Y = group_mul_hit(A, row0(rng.template propose_next<float>(a.delta, u)));
-      const float tY = group_retr(Y, M0);
-      const float dS = __fmul_rn(-bnc, __fsub_rn(tY, trO));
-      const bool down = dS < 0.f;
-      const bool accept = down || rng.accept(dS, u);
-      rng.advance(!down);
-      if (accept) {
-        A = Y;
-        trO = tY;
-        ++nacc;
+    for (int hit = 0; hit < a.nhits;) {
+      const int m = rng.ready(a.nhits - hit);
+      hit += m;
+#pragma unroll 1
+      for (int k = 0; k < m; ++k) {
+        const Row0<NC> Y = group_mul_hit(A, row0(rng.propose_next()));
+        const float tY = group_retr(Y, M0);
+        const float dS = __fmul_rn(-bnc, __fsub_rn(tY, trO));
+        const bool accept = rng.accept(dS);  // ln u <= 0: also of dS < 0
+        rng.advance(!(dS < 0.f));
+        if (accept) {
+          A = Y;
+          trO = tY;
+          ++nacc;
+        }
       }
     }
     if (nacc) {
@@ -559,24 +564,17 @@ struct GroupLaunch {
   cudaStream_t st = nullptr;
 };
 
+// The passes of a sweep after its first start before the kernel before them in the
+// stream, a pass of the same sweep, has ended.
 template <int NC, int ND, typename T, bool DF, int G> static cudaError_t launch_group_t(const GroupLaunch &l) {
   if (l.tab) {
-    multi_group_kernel<NC, ND, T, DF, G><<<l.blocks, GROUP_THREADS, 0, l.st>>>(*l.tab, l.val, l.nacc, l.slot);
-    return cudaGetLastError();
+    return launch_after(l.val > 0, multi_group_kernel<NC, ND, T, DF, G>, dim3(l.blocks), dim3(GROUP_THREADS), 0, l.st,
+                        *l.tab, l.val, l.nacc, l.slot);
   }
   const Geom &g = *l.g;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)group_blocks(g.Vh, G));
-  cfg.blockDim = dim3(GROUP_THREADS);
-  cfg.stream = l.st;
-  // the passes of a sweep after its first start before the one before has ended
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = l.val > 0 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, metropolis_group_kernel<NC, ND, T, DF, G>, Links<NC, T>{(cx<T> *)l.links, g.V}, g,
-                            l.val, *l.a, l.d_sweep, l.nacc, *l.df);
+  return launch_after(l.val > 0, metropolis_group_kernel<NC, ND, T, DF, G>, dim3((unsigned)group_blocks(g.Vh, G)),
+                      dim3(GROUP_THREADS), 0, l.st, Links<NC, T>{(cx<T> *)l.links, g.V}, g, l.val, *l.a, l.d_sweep,
+                      l.nacc, *l.df);
 }
 
 template <int NC, int ND, typename T> static cudaError_t launch_group_nd(int G, bool defect, const GroupLaunch &l) {
