@@ -210,6 +210,44 @@ __global__ void omega_kernel(Links<N, T> U, Geom g, ColGeom c, CField<N, T> om, 
   pol.store(col, O);
 }
 
+// The same with a column's rows in NSEG segments, one warp each (lanes over 32
+// columns): the segments' products, their prefix, then each segment walked from
+// its prefix.  Twice the products, but a chain of L_nu / NSEG + NSEG rows' loads and
+// products instead of L_nu (L_nu >= NSEG: a segment has a row).
+constexpr int OMEGA_SEG = 4;
+template <int N, typename T, int NSEG>
+__global__ void __launch_bounds__(32 * NSEG) omega_seg_kernel(Links<N, T> U, Geom g, ColGeom c, CField<N, T> om,
+                                                              CField<N, T> pol) {
+  __shared__ cx<double> P[NSEG - 1][N * N][32];
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const long long col = (long long)blockIdx.x * 32 + lane;
+  const bool ok = col < c.ncols;
+  const int b0 = c.Lnu * seg / NSEG, b1 = c.Lnu * (seg + 1) / NSEG;
+  int x[4];
+  col_coords(c, ok ? col : 0, x);
+  auto link = [&](int b) { return to_d(U.load(site_lin(g, col_site_at(c, x, b)), c.nu)); };
+  if (seg < NSEG - 1) {
+    Mat<N, double> O = link(b0);
+    for (int b = b0 + 1; b < b1; ++b) O = mul(O, link(b));
+#pragma unroll
+    for (int k = 0; k < N * N; ++k) P[seg][k][lane] = O.e[k / N][k % N];
+  }
+  __syncthreads();
+  if (!ok) return;
+  Mat<N, double> O = mident<N, double>();
+  for (int s = 0; s < seg; ++s) {
+    Mat<N, double> m;
+#pragma unroll
+    for (int k = 0; k < N * N; ++k) m.e[k / N][k % N] = P[s][k][lane];
+    O = s == 0 ? m : mul(O, m);
+  }
+  for (int b = b0; b < b1; ++b) {
+    om.store((long long)b * c.ncols + col, O);
+    O = mul(O, link(b));
+  }
+  if (seg == NSEG - 1) pol.store(col, O);
+}
+
 // U'_mu(col, row) for row < rows, over tiles of 32 consecutive columns x UP_RB
 // rows: computed with lanes over columns (coalesced U and Omega reads), staged
 // in shared memory and written column major (col * rows + row) with consecutive
@@ -819,7 +857,18 @@ static cudaError_t wilson_gf_t(const void *links, const Geom &g, const int *cons
   CField<N, T> pol{(cx<T> *)(base + al(es * Vc)), c[0].ncols};
   char *up0 = base + al(es * Vc) + al(es * c[0].ncols);
   Links<N, T> U{(cx<T> *)links, g.V};
-  if (!omega_ready) omega_kernel<N, T><<<(unsigned)((c[0].ncols + 127) / 128), 128, 0, st>>>(U, g, c[0], om, pol);
+  if (!omega_ready) {
+    // Four segments while the columns alone leave the device waiting on their chains:
+    // one temporal 1x1 loop of SU(3) FP64 16^3x32 81 -> 61 us, 24^3x48 255 -> 212, 8^4
+    // FP32 32.7 -> 30.7; at 32^3 columns SU(3) 313 -> 312 FP64, 154.6 -> 156.7 FP32 (the
+    // second product of each row), U(1) 64 -> 61, SU(2) 84 -> 74.  Eight segments gave
+    // no more.
+    const long long ncols = c[0].ncols;
+    if (c[0].Lnu >= OMEGA_SEG && (N < 3 || ncols < 24000))
+      omega_seg_kernel<N, T, OMEGA_SEG><<<(unsigned)((ncols + 31) / 32), 32 * OMEGA_SEG, 0, st>>>(U, g, c[0], om, pol);
+    else
+      omega_kernel<N, T><<<(unsigned)((ncols + 127) / 128), 128, 0, st>>>(U, g, c[0], om, pol);
+  }
   const long long nct = (c[0].ncols + 31) / 32;
   for (int i = 0; i < nplanes; ++i) {
     const CField<N, T> up{(cx<T> *)(up0 + i * up_bytes), c[i].ncols * c[i].rows};
