@@ -89,16 +89,17 @@ static cudaError_t launch_nd(int nd, void *links, const Geom &g, int val, const 
 // lane and form proposals that are not used, so they pay while the sites leave the
 // device idle.  us per sweep (4-D, nHits 10, FP64 | FP32), one thread per site
 // against a group:
-//   U(1)   8^4 497|463 -> 32 lanes 180|155, 12x8x10x20 497|466 -> 208|207,
+//   U(1)   8^4 497|463 -> 32 lanes 166|141, 12x8x10x20 497|466 -> 194|167,
 //          16^4 497|470 -> 16 lanes 368|286 (32: 450|412), 16^3x32 497|481, 16 lanes 652|558
-//   SU(2)  8^4 824|530 -> 32 lanes 241|200, 12x8x10x20 825|534 -> 370|285,
+//   SU(2)  8^4 824|530 -> 32 lanes 217|186, 12x8x10x20 825|534 -> 365|271,
 //          16^4 824|535 -> 16 lanes 725|465 (32: 746|577), 16^3x32 824|535, 16 lanes 1347|890
-//   SU(3)  8^4 1259|1382 -> 32 lanes 199|175, 12x8x10x20 1260|1388 -> 8 lanes 350|307
-//          (32: 440|268), 16^4 1259|1382 -> 499|443, 16^3x32 1265|1382 -> 973|781,
-//          24^4 1716|1647, 8 lanes 2219|1369
+//   SU(3)  8^4 1611|1486 -> 32 lanes 443|322, 12x8x10x20 1656|1502 -> 644|456 (8 lanes
+//          764|572), 16^4 1685|1517 -> 8 lanes 989|781, 16^3x32 1733|1527 -> 1697|1224,
+//          24^4 2232|1855, 8 lanes 3883|2402 (at the chain's own acceptance of 1 %; from
+//          a cold start, which accepts nothing, 8^4 199|175, 16^4 499|443)
 // A pass has V / 16 sites: 256, 1200, 4096, 8192, 20736.
 int group_lanes(int nc, int dtype, bool defect, long long sites) {
-  if (nc == 3) return sites <= 800 ? 32 : (sites <= (dtype == 0 ? 12000 : 24000) ? 8 : 1);
+  if (nc == 3) return sites <= 1500 ? 32 : (sites <= (dtype == 0 ? 8200 : 12000) ? 8 : 1);
   if (defect && dtype == 1) return 1;  // no FP32 form for U(1), SU(2) with a defect
   return sites <= 2048 ? 32 : (sites <= 5000 ? 16 : 1);
 }

@@ -13,11 +13,11 @@ DELTA = {1: 0.1, 2: 0.3, 3: 0.1}
 
 
 # sites per pass: a single one, ragged CTAs, either side of the changes of width
-# (800 and 2048); hits: none, one, more than a window of the stream holds
+# (1500 and 2048); hits: none, one, more than a window of the stream holds
 @pytest.mark.parametrize("nc,L,nhits", [(1, [2, 2], 3), (1, [6, 4], 1), (1, [4, 6, 10], 70), (1, [14, 16, 16, 16], 2),
                                         (2, [2, 2, 2], 5), (2, [4, 6, 8], 47), (2, [4, 4, 4, 6], 0),
                                         (2, [14, 16, 16, 16], 3), (3, [2, 4], 9), (3, [8, 6, 10, 4], 33),
-                                        (3, [10, 12, 12, 12], 11)])
+                                        (3, [12, 12, 12, 16], 11)])
 def test_group_pass_follows_oracle(oracle, nc, L, nhits):
     from oracle.oracle import Lat
     lat = Lat(nc, L)
