@@ -86,22 +86,30 @@ static cudaError_t launch_nd(int nd, void *links, const Geom &g, int val, const 
 }
 
 // More lanes shorten a site's chain of proposals but repeat its serial part in every
-// lane and form proposals that are not used, so they pay while the sites leave the
-// device idle.  us per sweep (4-D, nHits 10, FP64 | FP32), one thread per site
-// against a group:
-//   U(1)   8^4 497|463 -> 32 lanes 166|141, 12x8x10x20 497|466 -> 194|167,
-//          16^4 497|470 -> 16 lanes 368|286 (32: 450|412), 16^3x32 497|481, 16 lanes 652|558
-//   SU(2)  8^4 824|530 -> 32 lanes 217|186, 12x8x10x20 825|534 -> 365|271,
-//          16^4 824|535 -> 16 lanes 725|465 (32: 746|577), 16^3x32 824|535, 16 lanes 1347|890
-//   SU(3)  8^4 1611|1486 -> 32 lanes 443|322, 12x8x10x20 1656|1502 -> 644|456 (8 lanes
-//          764|572), 16^4 1685|1517 -> 8 lanes 989|781, 16^3x32 1733|1527 -> 1697|1224,
-//          24^4 2232|1855, 8 lanes 3883|2402 (at the chain's own acceptance of 1 %; from
-//          a cold start, which accepts nothing, 8^4 199|175, 16^4 499|443)
-// A pass has V / 16 sites: 256, 1200, 4096, 8192, 20736.
+// lane and form proposals that are not used, so fewer lanes pay as the sites fill
+// the device, and one thread per site once they do.  us per sweep (4-D, nHits 10) by
+// lanes, at 256, 1200, 2058, 4096, 8192 and 20736 sites a pass (V / 16):
+//   U(1) FP64   1: 511 527 529 530 529 561    32: 165 194 243 414 714 1780
+//               16: 190 202 206 281 505 1094   8: 212 216 220 237 319 868
+//   U(1) FP32   1: 464 480 476 470 480 528     8: 141 145 147 161 252 549
+//               4: 183 184 186 195 226 520
+//   SU(2) FP64  1: 824 842 857 842 836 981    32: 218 376 390 752 1469 3620
+//               16: 255 309 392 776 1228 2759
+//   SU(2) FP32  1: 505 529 530 530 529 617     8: 180 192 194 283 543 1036
+//               16: 177 192 206 318 603 1514
+// and SU(3) at 256, 1200, 4096, 8192, 20736 (at the chain's own acceptance of 1 %; a
+// cold start, which accepts nothing, takes half as long):
+//   SU(3) FP64  1: 1611 1656 1685 1733 2232   32: 443 644 1627 3016 7295
+//                8: 706 764 989 1697 3883
+//   SU(3) FP32  1: 1486 1502 1517 1527 1855   32: 322 456 1038 1992 5099
+//                8: 536 572 781 1224 2402
 int group_lanes(int nc, int dtype, bool defect, long long sites) {
-  if (nc == 3) return sites <= 1500 ? 32 : (sites <= (dtype == 0 ? 8200 : 12000) ? 8 : 1);
-  if (defect && dtype == 1) return 1;  // no FP32 form for U(1), SU(2) with a defect
-  return sites <= 2048 ? 32 : (sites <= 5000 ? 16 : 1);
+  const bool f64 = dtype == 0;
+  if (nc == 3) return sites <= 1500 ? 32 : (sites <= (f64 ? 8200 : 12000) ? 8 : 1);
+  if (defect && !f64) return 1;  // no FP32 form for U(1), SU(2) with a defect
+  if (nc == 2) return f64 ? (sites <= 1000 ? 32 : (sites <= 5500 ? 16 : 1)) : (sites <= 7500 ? 8 : 1);
+  if (f64) return sites <= 1300 ? 32 : (sites <= 2500 ? 16 : (sites <= 9000 ? 8 : 1));
+  return sites <= 6000 ? 8 : (sites <= 16000 ? 4 : 1);
 }
 
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,

@@ -40,7 +40,8 @@ template <int G> KLFT_D unsigned group_mask() {
 // Window of stream places in shared memory, per group.
 template <int NC, typename T, int G> struct DrawTable {
   static constexpr int K = RefDraws<NC>::n;
-  static constexpr int W = G == 32 ? (NC == 1 ? 96 : 160) : 32;
+  // 40 hits move on by 40-80 or 120-160 places: one window, or two, holds a site's
+  static constexpr int W = NC == 1 ? 96 : 160;
   static constexpr int N = W + K + 2;  // a hit looks up to K + 1 places past its own
   cx<T> prop[N][NC];  // row 0 of the proposal starting at each place
   double u[N];
@@ -577,15 +578,24 @@ template <int NC, int ND, typename T, bool DF, int G> static cudaError_t launch_
                       l.nacc, *l.df);
 }
 
+template <int NC, int ND, typename T, bool DF> static cudaError_t launch_group_df(int G, const GroupLaunch &l) {
+  // the widths group_lanes gives
+  if constexpr (NC == 3) return G == 32 ? launch_group_t<NC, ND, T, DF, 32>(l) : launch_group_t<NC, ND, T, DF, 8>(l);
+  else if constexpr (sizeof(T) == 4)
+    return NC == 1 && G == 4 ? launch_group_t<NC, ND, T, DF, (NC == 1 ? 4 : 8)>(l) : launch_group_t<NC, ND, T, DF, 8>(l);
+  else if constexpr (NC == 1)
+    return G == 32 ? launch_group_t<NC, ND, T, DF, 32>(l)
+                   : (G == 16 ? launch_group_t<NC, ND, T, DF, 16>(l) : launch_group_t<NC, ND, T, DF, 8>(l));
+  else return G == 32 ? launch_group_t<NC, ND, T, DF, 32>(l) : launch_group_t<NC, ND, T, DF, 16>(l);
+}
+
 template <int NC, int ND, typename T> static cudaError_t launch_group_nd(int G, bool defect, const GroupLaunch &l) {
-  constexpr int SMALL = NC == 3 ? 8 : 16;
   if constexpr (SharedStaples<NC, T>::v) {
-    if (defect)
-      return G == 32 ? launch_group_t<NC, ND, T, true, 32>(l) : launch_group_t<NC, ND, T, true, SMALL>(l);
+    if (defect) return launch_group_df<NC, ND, T, true>(G, l);
   } else {
     if (defect) return cudaErrorInvalidValue;  // group_lanes gives 1
   }
-  return G == 32 ? launch_group_t<NC, ND, T, false, 32>(l) : launch_group_t<NC, ND, T, false, SMALL>(l);
+  return launch_group_df<NC, ND, T, false>(G, l);
 }
 
 template <int NC> static cudaError_t launch_group_nc(int nd, int dtype, int G, bool defect, const GroupLaunch &l) {
