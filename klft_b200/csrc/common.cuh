@@ -123,6 +123,24 @@ template <typename T> KLFT_HD cx<T> operator-(cx<T> a, cx<T> b) { return {a.re -
 template <typename T> KLFT_HD cx<T> operator*(cx<T> a, cx<T> b) {
   return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 }
+// FP64 on the device: the same arithmetic with its FMAs written out.  The compiler
+// contracts a b - c d by the order in which it finds the operands, which differs
+// from kernel to kernel; so a chain is the same bit for bit whichever pass kernel
+// (one thread per site, a group of lanes, alone or in a batch) its size selects.
+KLFT_HD cx<double> operator*(cx<double> a, cx<double> b) {
+#ifdef __CUDA_ARCH__
+  return {fma(a.re, b.re, -__dmul_rn(a.im, b.im)), fma(a.re, b.im, __dmul_rn(a.im, b.re))};
+#else
+  return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
+#endif
+}
+// |a|^2, and s + |a|^2, contracted one way in FP64
+template <typename T> KLFT_HD T norm2(cx<T> a) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(T) == 8) return fma(a.re, a.re, __dmul_rn(a.im, a.im));
+#endif
+  return a.re * a.re + a.im * a.im;
+}
 template <typename T> KLFT_HD cx<T> operator*(cx<T> a, T s) { return {a.re * s, a.im * s}; }
 template <typename T> KLFT_HD cx<T> operator*(T s, cx<T> a) { return {s * a.re, s * a.im}; }
 template <typename T> KLFT_HD cx<T> conj(cx<T> a) { return {a.re, -a.im}; }
@@ -314,7 +332,7 @@ template <int N, typename T, typename A> KLFT_HD A retr_nd(const Mat<N, T> &a, c
 // restoreSUN (SUN.hpp:256-340)
 template <typename T> KLFT_HD Mat<1, T> restore(const Mat<1, T> &a) {
   Mat<1, T> c;
-  const T n = sqrt(a.e[0][0].re * a.e[0][0].re + a.e[0][0].im * a.e[0][0].im);
+  const T n = sqrt(norm2(a.e[0][0]));
   if constexpr (sizeof(T) == 4) {
     const T i = T(1) / n;  // FP32: one reciprocal (see the SU(3) form)
     c.e[0][0] = mk<T>(a.e[0][0].re * i, a.e[0][0].im * i);
@@ -325,8 +343,11 @@ template <typename T> KLFT_HD Mat<1, T> restore(const Mat<1, T> &a) {
 }
 template <typename T> KLFT_HD Mat<2, T> restore(const Mat<2, T> &a) {
   Mat<2, T> c;
-  const T n = sqrt(a.e[0][0].re * a.e[0][0].re + a.e[0][0].im * a.e[0][0].im + a.e[0][1].re * a.e[0][1].re +
-                   a.e[0][1].im * a.e[0][1].im);
+  T n;
+  if constexpr (sizeof(T) == 8) n = sqrt(norm2(a.e[0][0]) + norm2(a.e[0][1]));
+  else
+    n = sqrt(a.e[0][0].re * a.e[0][0].re + a.e[0][0].im * a.e[0][0].im + a.e[0][1].re * a.e[0][1].re +
+             a.e[0][1].im * a.e[0][1].im);
   if constexpr (sizeof(T) == 4) {
     const T r = T(1) / n;  // FP32: one reciprocal (see the SU(3) form)
 #pragma unroll
