@@ -310,7 +310,7 @@ cudaError_t launch_group_nc(const GroupKey &k, const ChainTable &tab, int blocks
   return launch_group_nd<NC, 4, T>(k, tab, blocks, val, nacc, slot, st);
 }
 
-// lanes > 1: the reference-proposal pass by groups of lanes (metropolis_group.cuh)
+// lanes > 1: the pass by groups of lanes (metropolis_group.cuh, metropolis_exp_group.cuh)
 cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, int lanes, int val,
                          unsigned long long *nacc, const uint32_t *slot, cudaStream_t st) {
   if (lanes > 1) {
@@ -321,6 +321,7 @@ cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, i
     l.val = val;
     l.nacc = nacc;
     l.st = st;
+    if (k.exp) return k.dtype == 0 ? launch_exp_group_f64(k.nd, lanes, k.df, l) : launch_exp_group_f32(k.nd, lanes, k.df, l);
     if (k.nc == 1) return launch_group_u1(k.nd, k.dtype, lanes, k.df, l);
     if (k.nc == 2) return launch_group_su2(k.nd, k.dtype, lanes, k.df, l);
     return launch_group_su3(k.nd, k.dtype, lanes, k.df, l);
@@ -338,7 +339,7 @@ cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, i
 struct Group {
   GroupKey key;
   long long sites = 0;  // of one pass, all chains
-  int lanes = 1;        // per site (reference proposals)
+  int lanes = 1;        // per site, or per link of the exp proposal
   std::vector<std::unique_ptr<ChainTable>> tables;
   std::vector<int> blocks;
 };
@@ -371,7 +372,8 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
   };
   for (const SweepItem &it : items) group_of(key_of(it)).sites += it.lat->g.Vh;
   for (auto &gg : groups)
-    if (!gg.key.exp) gg.lanes = group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
+    gg.lanes = gg.key.exp ? exp_group_lanes(gg.key.dtype, gg.key.df, gg.sites << (gg.key.nd - 1))
+                          : group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
   for (int i = 0; i < n; ++i) {
     const SweepItem &it = items[i];
     klft_lattice *lat = it.lat;
@@ -397,7 +399,7 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
     d.block_begin = grp->blocks.back();
     // exp groups: V/2 links per link pass; reference groups: Vh sites per class
     const long long nthr = key.exp ? link_pass_threads(lat->g, lat->g.nd) : lat->g.Vh;
-    grp->blocks.back() += grp->lanes > 1 ? (int)group_blocks(lat->g.Vh, grp->lanes) : (int)((nthr + block - 1) / block);
+    grp->blocks.back() += grp->lanes > 1 ? (int)group_blocks(nthr, grp->lanes) : (int)((nthr + block - 1) / block);
   }
   int maxpass = 0;
   for (auto &gg : groups) {

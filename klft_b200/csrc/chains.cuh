@@ -34,4 +34,23 @@ KLFT_D int find_chain(const ChainTable &tab) {
   return lo;
 }
 
+// One pass by groups of lanes, of one lattice or of many chains.
+struct GroupLaunch {
+  // one lattice
+  void *links = nullptr;
+  const Geom *g = nullptr;
+  const MetroArgs *a = nullptr;
+  const Defect *df = nullptr;
+  const uint32_t *d_sweep = nullptr;
+  // many chains
+  const ChainTable *tab = nullptr;
+  int blocks = 0;
+  const uint32_t *slot = nullptr;
+  int val = 0;
+  unsigned long long *nacc = nullptr;
+  cudaStream_t st = nullptr;
+};
+cudaError_t launch_exp_group_f32(int nd, int G, bool defect, const GroupLaunch &l);
+cudaError_t launch_exp_group_f64(int nd, int G, bool defect, const GroupLaunch &l);
+
 }  // namespace klft

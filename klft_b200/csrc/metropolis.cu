@@ -112,21 +112,37 @@ int group_lanes(int nc, int dtype, bool defect, long long sites) {
   return sites <= 6000 ? 8 : (sites <= 16000 ? 4 : 1);
 }
 
+// The chain of a link's accepted products is repeated in every lane, so groups pay
+// while the links leave the device idle.  us per sweep (4-D, nHits 10) by lanes, at
+// 128, 2048, 3200, 4800 and 9600 links a pass (V / 2):
+//   FP64  1: 169 184 185 184 185   4: 106 109 119 131 220   16: 78 106 183 252 424
+//   FP32  1: 132 134 133 132 134   4:  90  93 102 108 166   16: 63  78 103 163 253
+// (3-D, 840 links: FP64 127, 73, 66; FP32 91, 60, 52.)  FP32 links with a defect keep
+// one thread: their staple's contraction, and with it the chain's bits, differ here.
+int exp_group_lanes(int dtype, bool defect, long long links) {
+  if (defect && dtype == 1) return 1;
+  return links <= 2500 ? 16 : (links <= 6500 ? 4 : 1);
+}
+
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,
                                    const uint32_t *d_sweep, unsigned long long *d_nacc, const Defect &df, int block,
                                    cudaStream_t st) {
   const bool exp = nc == 3 && a.proposal == PROPOSAL_EXP;
-  const int lanes = exp ? 1 : group_lanes(nc, dtype, df.active != 0, g.Vh);
+  const int lanes = exp ? exp_group_lanes(dtype, df.active != 0, g.V / 2) : group_lanes(nc, dtype, df.active != 0, g.Vh);
   if (lanes > 1) {
+    MetroArgs b = a;
+    // the FP64 exp(i eps H) proposal reads its Gaussians from the host-built table
+    if (exp && dtype == 0 && !(b.bm = bm_table())) return cudaErrorMemoryAllocation;
     GroupLaunch l;
     l.links = links;
     l.g = &g;
-    l.a = &a;
+    l.a = &b;
     l.df = &df;
     l.d_sweep = d_sweep;
     l.val = val;
     l.nacc = d_nacc;
     l.st = st;
+    if (exp) return dtype == 0 ? launch_exp_group_f64(g.nd, lanes, df.active != 0, l) : launch_exp_group_f32(g.nd, lanes, df.active != 0, l);
     if (nc == 1) return launch_group_u1(g.nd, dtype, lanes, df.active != 0, l);
     if (nc == 2) return launch_group_su2(g.nd, dtype, lanes, df.active != 0, l);
     return launch_group_su3(g.nd, dtype, lanes, df.active != 0, l);

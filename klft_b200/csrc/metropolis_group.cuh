@@ -548,23 +548,6 @@ __global__ void __launch_bounds__(GROUP_THREADS)
               nacc_slots + (size_t)(*slot) * tab.nchains_total + c.index);
 }
 
-// One launch of either kind.
-struct GroupLaunch {
-  // one lattice
-  void *links = nullptr;
-  const Geom *g = nullptr;
-  const MetroArgs *a = nullptr;
-  const Defect *df = nullptr;
-  const uint32_t *d_sweep = nullptr;
-  // many chains
-  const ChainTable *tab = nullptr;
-  int blocks = 0;
-  const uint32_t *slot = nullptr;
-  int val = 0;
-  unsigned long long *nacc = nullptr;
-  cudaStream_t st = nullptr;
-};
-
 // The passes of a sweep after its first start before the kernel before them in the
 // stream, a pass of the same sweep, has ended.
 template <int NC, int ND, typename T, bool DF, int G> static cudaError_t launch_group_t(const GroupLaunch &l) {

@@ -1,6 +1,6 @@
-"""Reference-proposal passes by groups of lanes (small lattices): the same chain as
-the oracle's and as the pass with one thread per site, which a batch takes when
-its other chains make the launch large."""
+"""Passes by groups of lanes (small lattices): the same chain as the oracle's and as
+the pass with one thread per site or link, which a batch takes when its other chains
+make the launch large."""
 import numpy as np
 import pytest
 
@@ -52,5 +52,29 @@ def test_group_pass_is_the_chain_of_the_site_pass(nc, precision, L, defect):
         b.add(g, BETA[nc], DELTA[nc], 10)
     acc, _, _, _ = b.run(3, False, False)
     np.testing.assert_array_equal(alone.metropolis(BETA[nc], DELTA[nc], 10, 3), acc[:, 0])
+    np.testing.assert_array_equal(alone.download(), member.download())
+    b.close()
+
+
+# 16 lanes, 4 lanes, 3 and 2 dimensions; hits: fewer and more than the lanes
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("L,defect,nhits", [([8, 6, 4, 10], 0, 10), ([8, 6, 4, 10], 2, 37), ([8, 8, 8, 16], 0, 10),
+                                            ([8, 8, 8, 16], 2, 6), ([10, 12, 14], 0, 37), ([20, 14], 0, 1)])
+def test_exp_group_pass_is_the_chain_of_the_link_pass(precision, L, defect, nhits):
+    big = [16, 16, 16, 8] if len(L) == 4 else ([32, 32, 16] if len(L) == 3 else [128, 128])
+
+    def field(ext, seed):
+        g = GaugeField(ext, 3, precision, "hot", seed)
+        g.set_stream(seed, 1)
+        if defect:
+            g.set_defect(defect, (0, 1, 0), 0.5)
+        return g
+
+    alone, member, other = field(L, 5), field(L, 5), field(big, 6)
+    b = Batch()
+    for g in (member, other):
+        b.add(g, 5.7, 0.0, nhits, "exp", 0.25)
+    acc, _, _, _ = b.run(3, False, False)
+    np.testing.assert_array_equal(alone.metropolis(5.7, 0.0, nhits, 3, "exp", 0.25), acc[:, 0])
     np.testing.assert_array_equal(alone.download(), member.download())
     b.close()
