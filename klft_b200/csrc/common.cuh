@@ -134,7 +134,11 @@ KLFT_HD cx<double> operator*(cx<double> a, cx<double> b) {
   return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 #endif
 }
-// |a|^2, and s + |a|^2, contracted one way in FP64
+// a * b as the compiler contracts it
+template <typename T> KLFT_HD cx<T> cmul_plain(cx<T> a, cx<T> b) {
+  return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
+}
+// |a|^2, contracted one way in FP64
 template <typename T> KLFT_HD T norm2(cx<T> a) {
 #ifdef __CUDA_ARCH__
   if constexpr (sizeof(T) == 8) return fma(a.re, a.re, __dmul_rn(a.im, a.im));
@@ -385,6 +389,44 @@ template <typename T> KLFT_HD Mat<3, T> restore(const Mat<3, T> &a) {
   c.e[1][0] = conj(c.e[2][1] * c.e[0][2] - c.e[2][2] * c.e[0][1]);
   c.e[1][1] = conj(c.e[2][2] * c.e[0][0] - c.e[2][0] * c.e[0][2]);
   c.e[1][2] = conj(c.e[2][0] * c.e[0][1] - c.e[2][1] * c.e[0][0]);
+  return c;
+}
+
+// The same in FP64 for links stored in FP32, in the compiler's contraction: the last
+// bit of an FP64 value decides one FP32 rounding in 10^9, and the mixed form's fields
+// are to keep theirs.
+KLFT_HD Mat<1, double> restore_plain(const Mat<1, double> &a) {
+  Mat<1, double> c;
+  const double n = sqrt(a.e[0][0].re * a.e[0][0].re + a.e[0][0].im * a.e[0][0].im);
+  c.e[0][0] = cdiv(a.e[0][0], n);
+  return c;
+}
+KLFT_HD Mat<2, double> restore_plain(const Mat<2, double> &a) {
+  Mat<2, double> c;
+  const double n = sqrt(a.e[0][0].re * a.e[0][0].re + a.e[0][0].im * a.e[0][0].im + a.e[0][1].re * a.e[0][1].re +
+                        a.e[0][1].im * a.e[0][1].im);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) c.e[i][j] = cdiv(a.e[i][j], n);
+  return c;
+}
+KLFT_HD Mat<3, double> restore_plain(const Mat<3, double> &a) {
+  Mat<3, double> c;
+  auto p = [](cx<double> x, cx<double> y) { return cmul_plain(x, y); };
+  const double n0 = sqrt((p(conj(a.e[0][0]), a.e[0][0]) + p(conj(a.e[0][1]), a.e[0][1]) + p(conj(a.e[0][2]), a.e[0][2])).re);
+  const double n1 = sqrt((p(conj(a.e[1][0]), a.e[1][0]) + p(conj(a.e[1][1]), a.e[1][1]) + p(conj(a.e[1][2]), a.e[1][2])).re);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    c.e[0][j] = cdiv(a.e[0][j], n0);
+    c.e[1][j] = cdiv(a.e[1][j], n1);
+  }
+  c.e[2][0] = conj(p(c.e[0][1], c.e[1][2]) - p(c.e[0][2], c.e[1][1]));
+  c.e[2][1] = conj(p(c.e[0][2], c.e[1][0]) - p(c.e[0][0], c.e[1][2]));
+  c.e[2][2] = conj(p(c.e[0][0], c.e[1][1]) - p(c.e[0][1], c.e[1][0]));
+  c.e[1][0] = conj(p(c.e[2][1], c.e[0][2]) - p(c.e[2][2], c.e[0][1]));
+  c.e[1][1] = conj(p(c.e[2][2], c.e[0][0]) - p(c.e[2][0], c.e[0][2]));
+  c.e[1][2] = conj(p(c.e[2][0], c.e[0][1]) - p(c.e[2][1], c.e[0][0]));
   return c;
 }
 

@@ -106,7 +106,7 @@ __global__ void reunitarize_kernel(Links<NC, T> U, Geom g) {
   for (int i = 0; i < NC; ++i)
 #pragma unroll
     for (int j = 0; j < NC; ++j) d.e[i][j] = mk<double>((double)m.e[i][j].re, (double)m.e[i][j].im);
-  d = restore(d);
+  d = restore_plain(d);
   Mat<NC, T> o;
 #pragma unroll
   for (int i = 0; i < NC; ++i)

@@ -139,17 +139,19 @@ template <typename T> KLFT_D Mat<3, T> haar(Stream &g, const Mat<3, T> *) {
                          r0[2].re * r0[2].re + r0[2].im * r0[2].im);
 #pragma unroll
   for (int j = 0; j < 3; ++j) r0[j] = cdiv(r0[j], n0);
-  const cx<double> z = conj(r0[0]) * r1[0] + conj(r0[1]) * r1[1] + conj(r0[2]) * r1[2];
+  // products in the compiler's contraction (restore_plain)
+  auto p = [](cx<double> x, cx<double> y) { return cmul_plain(x, y); };
+  const cx<double> z = p(conj(r0[0]), r1[0]) + p(conj(r0[1]), r1[1]) + p(conj(r0[2]), r1[2]);
 #pragma unroll
-  for (int j = 0; j < 3; ++j) r1[j] -= z * r0[j];
+  for (int j = 0; j < 3; ++j) r1[j] -= p(z, r0[j]);
   const double n1 = sqrt(r1[0].re * r1[0].re + r1[0].im * r1[0].im + r1[1].re * r1[1].re + r1[1].im * r1[1].im +
                          r1[2].re * r1[2].re + r1[2].im * r1[2].im);
 #pragma unroll
   for (int j = 0; j < 3; ++j) r1[j] = cdiv(r1[j], n1);
   cx<double> r2[3];
-  r2[0] = conj(r0[1] * r1[2] - r0[2] * r1[1]);
-  r2[1] = conj(r0[2] * r1[0] - r0[0] * r1[2]);
-  r2[2] = conj(r0[0] * r1[1] - r0[1] * r1[0]);
+  r2[0] = conj(p(r0[1], r1[2]) - p(r0[2], r1[1]));
+  r2[1] = conj(p(r0[2], r1[0]) - p(r0[0], r1[2]));
+  r2[2] = conj(p(r0[0], r1[1]) - p(r0[1], r1[0]));
   Mat<3, T> m;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
