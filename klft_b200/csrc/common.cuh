@@ -359,10 +359,10 @@ template <typename T> KLFT_HD Mat<2, T> restore(const Mat<2, T> &a) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) c.e[i][j] = mk<T>(a.e[i][j].re * r, a.e[i][j].im * r);
   } else {
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) c.e[i][j] = cdiv(a.e[i][j], n);
+    // a is a product, row 1 the conjugate of row 0: four divisions give all eight values
+    c.e[0][0] = cdiv(a.e[0][0], n);
+    c.e[0][1] = cdiv(a.e[0][1], n);
+    su2_row1(c);
   }
   return c;
 }

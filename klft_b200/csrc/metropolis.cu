@@ -6,7 +6,8 @@
 // enqueues one launch per class.  Sites of one class share no staple link, so
 // a pass is race free.  exp(i eps H) proposals: 2 Nd link passes (mu, parity)
 // of one thread per link (metropolis_site.cuh).  The per-site and per-link
-// updates are in metropolis_site.cuh.
+// updates are in metropolis_site.cuh.  Passes too small to fill the device so go
+// to groups of lanes (metropolis_group.cuh, metropolis_exp_group.cuh).
 #include "metropolis_group.cuh"
 
 namespace klft {
