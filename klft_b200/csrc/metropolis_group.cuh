@@ -258,6 +258,9 @@ template <bool FIRST> KLFT_D Row0<2> group_new_link(const Row0<2> &u, const Row0
   const float i = 1.0f / sqrtf(fmaf(q.im, q.im, fmaf(q.re, q.re, mad2(p.re, p.re, p.im, p.im))));
   return {{mk<float>(__fmul_rn(p.re, i), __fmul_rn(p.im, i)), mk<float>(__fmul_rn(q.re, i), __fmul_rn(q.im, i))}};
 }
+// Every lane runs the hits on the link and the staple as it loaded them, so lane 0
+// stores the new link between two barriers: no lane then reads it half way, and the
+// next direction's staple sees it.
 template <int NC, int ND, int MU, typename Draws>
 KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &x, const MetroArgs &a, Draws &rng) {
   if constexpr (MU < ND) {
@@ -292,7 +295,9 @@ KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &
       Mat<NC, float> m;
 #pragma unroll
       for (int j = 0; j < NC; ++j) m.e[0][j] = V.v[j];
-      U.store(lx, MU, m);
+      __syncwarp(rng.mask);
+      if (rng.gl == 0) U.store(lx, MU, m);
+      __syncwarp(rng.mask);
     }
     return nacc;
   }
@@ -511,9 +516,10 @@ KLFT_D int group_site_update(GroupShared<NC, ND, T, G> *shared, const Links<NC, 
           return group_hits<NC, T>(S, V, a, dlink, df, rng, bnc);
         });
       } else {
-        // every lane: the same links, decisions and stores
+        // every lane: the same links and decisions
         static_assert(!DF, "FP32 U(1), SU(2): lattices without a defect");
         touch_neighbours<NC, ND, T, G>(U, g, x, gl);
+        __syncwarp(rng.mask);
         n = group_link_f32<NC, ND, 0>(U, g, x, a, rng);
         n += group_link_f32<NC, ND, 1>(U, g, x, a, rng);
         n += group_link_f32<NC, ND, 2>(U, g, x, a, rng);

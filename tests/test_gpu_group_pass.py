@@ -78,3 +78,27 @@ def test_exp_group_pass_is_the_chain_of_the_link_pass(precision, L, defect, nhit
     np.testing.assert_array_equal(alone.metropolis(5.7, 0.0, nhits, 3, "exp", 0.25), acc[:, 0])
     np.testing.assert_array_equal(alone.download(), member.download())
     b.close()
+
+
+# FP32 U(1) and SU(2), where each lane runs the site's hits on links that lane 0 stores:
+# one site to several CTAs, 4 and 8 lanes, hits that need no window, one, and several
+# (so that a link's hits are resumed in a new window), and extents that leave the lanes
+# of a group with different shares of the neighbours
+@pytest.mark.parametrize("nc", [1, 2])
+@pytest.mark.parametrize("L,nhits", [([2, 2], 47), ([6, 4], 11), ([4, 6, 10], 0), ([4, 6, 10], 47), ([2, 2, 2], 30),
+                                     ([6, 2, 4, 2], 1), ([4, 4, 4, 6], 11), ([8, 6, 4, 10], 47), ([40, 44, 48], 11)])
+def test_fp32_group_pass_resumes_hits_and_orders_stores(nc, L, nhits):
+    big = {4: [24, 24, 24, 32], 3: [64, 56, 56], 2: [320, 320]}[len(L)]
+    fields = []
+    for ext, seed in ((L, 5), (L, 5), (big, 6)):
+        g = GaugeField(ext, nc, "mixed", "hot", seed)
+        g.set_stream(seed, 1)
+        fields.append(g)
+    alone, member, other = fields
+    b = Batch()
+    for g in (member, other):
+        b.add(g, BETA[nc], DELTA[nc], nhits)
+    acc, _, _, _ = b.run(4, False, False)
+    np.testing.assert_array_equal(alone.metropolis(BETA[nc], DELTA[nc], nhits, 4), acc[:, 0])
+    np.testing.assert_array_equal(alone.download(), member.download())
+    b.close()
