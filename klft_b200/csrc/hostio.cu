@@ -49,7 +49,9 @@ size_t chunk_bytes(size_t total) {
   return std::min<size_t>(4u << 20, std::max<size_t>(1u << 20, c));
 }
 
-// A small persistent pool of host threads for the staging memcpys.
+// A small persistent pool of host threads for the staging memcpys.  It works on one
+// job at a time: transfers on two devices, whose staging buffers have a lock each,
+// take turns on it (a job of theirs fills all threads).
 class CopyPool {
  public:
   static CopyPool &get() {
@@ -62,6 +64,7 @@ class CopyPool {
       for (int i = 0; i < n; ++i) fn(i);
       return;
     }
+    std::lock_guard<std::mutex> job(job_mu_);
     std::unique_lock<std::mutex> lk(mu_);
     fn_ = &fn;
     next_ = 0;
@@ -119,7 +122,8 @@ class CopyPool {
     }
   }
   std::vector<std::thread> workers_;
-  std::mutex mu_;
+  std::mutex job_mu_;  // held for the whole of a job
+  std::mutex mu_;      // the job's state
   std::condition_variable cv_, done_cv_;
   const std::function<void(int)> *fn_ = nullptr;
   int next_ = 0, n_ = 0, done_ = 0;
