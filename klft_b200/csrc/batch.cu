@@ -349,6 +349,27 @@ GroupKey key_of(const klft::SweepItem &it) {
                   (it.lat->nc == 3 && it.a.proposal == KLFT_PROPOSAL_EXP) ? 1 : 0, it.df.active ? 1 : 0};
 }
 
+// the launch groups of the items and their lanes, no chains yet
+std::vector<Group> groups_of(const std::vector<klft::SweepItem> &items) {
+  std::vector<Group> groups;
+  for (const klft::SweepItem &it : items) {
+    const GroupKey key = key_of(it);
+    Group *grp = nullptr;
+    for (auto &gg : groups)
+      if (gg.key == key) grp = &gg;
+    if (!grp) {
+      groups.emplace_back();
+      grp = &groups.back();
+      grp->key = key;
+    }
+    grp->sites += it.lat->g.Vh;
+  }
+  for (auto &gg : groups)
+    gg.lanes = gg.key.exp ? exp_group_lanes(gg.key.dtype, gg.key.df, gg.sites << (gg.key.nd - 1))
+                          : group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
+  return groups;
+}
+
 }  // namespace
 
 namespace klft {
@@ -362,23 +383,14 @@ klft_status enqueue_multi_sweep(const std::vector<SweepItem> &items, unsigned lo
   if (block != 32 && block != 64 && block != 128) return fail(KLFT_EINVAL, "enqueue_multi_sweep: block %d", block);
   const int n = (int)items.size();
   const int stride = acc_stride > 0 ? acc_stride : n;
-  std::vector<Group> groups;
-  auto group_of = [&](const GroupKey &key) -> Group & {
-    for (auto &gg : groups)
-      if (gg.key == key) return gg;
-    groups.emplace_back();
-    groups.back().key = key;
-    return groups.back();
-  };
-  for (const SweepItem &it : items) group_of(key_of(it)).sites += it.lat->g.Vh;
-  for (auto &gg : groups)
-    gg.lanes = gg.key.exp ? exp_group_lanes(gg.key.dtype, gg.key.df, gg.sites << (gg.key.nd - 1))
-                          : group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
+  std::vector<Group> groups = groups_of(items);
   for (int i = 0; i < n; ++i) {
     const SweepItem &it = items[i];
     klft_lattice *lat = it.lat;
     const GroupKey key = key_of(it);
-    Group *grp = &group_of(key);
+    Group *grp = nullptr;
+    for (auto &gg : groups)
+      if (gg.key == key) grp = &gg;
     if (grp->tables.empty() || grp->tables.back()->n == BATCH_MAX) {
       grp->tables.emplace_back(new ChainTable());
       std::memset(grp->tables.back().get(), 0, sizeof(ChainTable));
@@ -540,6 +552,13 @@ klft_status tune_sweep_block(klft_batch *b) {
   const int end[1] = {(int)std::min<long long>(sites, 2147483647LL)};
   const std::string key = tune_key(id, 1, end);
   const std::vector<SweepItem> items = sweep_items(b);
+  // passes by groups of lanes have one launch shape: nothing to time
+  bool sized = false;
+  for (const Group &gg : groups_of(items)) sized = sized || gg.lanes == 1;
+  if (!sized) {
+    b->sweep_block = tuned_param(key, 1, {128}, 128, [](int) { return 0.f; }, true);
+    return KLFT_OK;
+  }
   auto time_fn = [&](int block) -> float {
     if (b->s_tune.ensure(total) != cudaSuccess) return -1.f;
     char *bak = (char *)b->s_tune.ptr;

@@ -767,13 +767,16 @@ klft_status klft_run_metropolis(klft_lattice *lat, double beta, double delta, in
 namespace klft {
 
 // Block size of the sweep passes: 128 unless the tuner (KLFT_TUNING) picked
-// another; candidates are timed on a scratch copy of the links.
+// another; candidates are timed on a scratch copy of the links.  Passes by groups
+// of lanes have one launch shape: their key is kept with it and nothing is timed.
 static int sweep_block(klft_lattice *lat, const MetroArgs &a, const Defect &df, bool may_tune) {
   if (!tuner_enabled()) return 128;
   const std::string id = std::string("sweep_Metropolis_GaugeField_nc") + std::to_string(lat->nc) +
                          (lat->dtype() == 0 ? "_fp64" : "_mixed") +
                          (a.proposal == KLFT_PROPOSAL_EXP && lat->nc == 3 ? "_exp" : "_ref");
   const std::string key = tune_key(id, lat->g.nd, lat->g.H);
+  if (pass_lanes(lat->nc, lat->dtype(), a.proposal, df.active != 0, lat->g) > 1)
+    return tuned_param(key, lat->g.nd, {128}, 128, [](int) { return 0.f; }, may_tune);
   auto time_fn = [&](int block) -> float {
     const size_t off = (lat->link_bytes + 255) & ~(size_t)255;
     if (lat->s_tune.ensure(off + 256) != cudaSuccess) return -1.f;

@@ -27,6 +27,8 @@ KLFT_HD int metropolis_passes(int nc, int proposal, int nd) { return nc == 3 && 
 int group_lanes(int nc, int dtype, bool defect, long long sites);
 // The SU(3) exp proposal: lanes per link of a pass over `links` links.
 int exp_group_lanes(int dtype, bool defect, long long links);
+// What one of the two gives for a pass of one lattice (proposal as in MetroArgs).
+int pass_lanes(int nc, int dtype, int proposal, bool defect, const Geom &g);
 constexpr int GROUP_THREADS = 64;  // per CTA of the group kernels: few sites over many SMs
 inline long long group_blocks(long long sites, int lanes) { return (sites * lanes + GROUP_THREADS - 1) / GROUP_THREADS; }
 

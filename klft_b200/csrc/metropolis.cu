@@ -125,11 +125,16 @@ int exp_group_lanes(int dtype, bool defect, long long links) {
   return links <= 2500 ? 16 : (links <= 6500 ? 4 : 1);
 }
 
+int pass_lanes(int nc, int dtype, int proposal, bool defect, const Geom &g) {
+  if (nc == 3 && proposal == PROPOSAL_EXP) return exp_group_lanes(dtype, defect, g.V / 2);
+  return group_lanes(nc, dtype, defect, g.Vh);
+}
+
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,
                                    const uint32_t *d_sweep, unsigned long long *d_nacc, const Defect &df, int block,
                                    cudaStream_t st) {
   const bool exp = nc == 3 && a.proposal == PROPOSAL_EXP;
-  const int lanes = exp ? exp_group_lanes(dtype, df.active != 0, g.V / 2) : group_lanes(nc, dtype, df.active != 0, g.Vh);
+  const int lanes = pass_lanes(nc, dtype, a.proposal, df.active != 0, g);
   if (lanes > 1) {
     MetroArgs b = a;
     // the FP64 exp(i eps H) proposal reads its Gaussians from the host-built table
