@@ -155,7 +155,8 @@ template <typename T> KLFT_HD void operator-=(cx<T> &a, cx<T> b) { a.re -= b.re;
 // quarter fewer FP64 instructions so, and those kernels are bound by them (pipe and
 // latency): a link pass of the FP64 exp proposal, 16^3x32, executed 5.7 M FMAs
 // beside 6.9 M other FP64 instructions.  FP32 keeps the compiler's form, and with it
-// the bits of the mixed form's chains.
+// the bits of the mixed form's chains.  Such a chain rounds twice per term at the size
+// of the sum so far, so the products below take their largest term last (sum_term).
 template <typename T> KLFT_HD void cmac(cx<T> &s, cx<T> a, cx<T> b) {
 #ifdef __CUDA_ARCH__
   if constexpr (sizeof(T) == 8) {
@@ -186,6 +187,14 @@ template <int N, typename T> KLFT_HD Mat<N, T> mident() {
   for (int i = 0; i < N; ++i) m.e[i][i] = mk<T>(T(1), T(0));
   return m;
 }
+// The k of the n-th term of sum_k a_ik b_kj.  SU(3) in FP64: the diagonal elements, the
+// large ones except at strong coupling, have k = i last.  RMS error of a product of
+// links of spread 0.15 about the identity: 1.98e-17, with k in order 2.76e-17 (2.65e-17
+// without cmac's chain); of Haar-random links 3.60e-17 in both (3.54e-17).
+template <int N, typename T> KLFT_HD constexpr int sum_term(int i, int j, int n) {
+  if (sizeof(T) == 4 || N < 3 || i != j) return n;
+  return n == 2 ? i : (n < i ? n : n + 1);
+}
 // SU(2) elements, and real combinations of them (staple sums, algebra
 // elements), have the form [[x, y], [-conj(y), conj(x)]]; so does every product
 // of two of them.  The products below form row 0 (in the general order) and
@@ -208,9 +217,13 @@ template <int N, typename T> KLFT_HD Mat<N, T> mul(const Mat<N, T> &a, const Mat
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<T> s = a.e[i][0] * b.e[0][j];
+      const int k0 = sum_term<N, T>(i, j, 0);
+      cx<T> s = a.e[i][k0] * b.e[k0][j];
 #pragma unroll
-      for (int k = 1; k < N; ++k) cmac(s, a.e[i][k], b.e[k][j]);
+      for (int n = 1; n < N; ++n) {
+        const int k = sum_term<N, T>(i, j, n);
+        cmac(s, a.e[i][k], b.e[k][j]);
+      }
       c.e[i][j] = s;
     }
   return c;
@@ -228,9 +241,13 @@ template <int N, typename T> KLFT_HD Mat<N, T> mul_nd(const Mat<N, T> &a, const 
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<T> s = a.e[i][0] * conj(b.e[j][0]);
+      const int k0 = sum_term<N, T>(i, j, 0);
+      cx<T> s = a.e[i][k0] * conj(b.e[j][k0]);
 #pragma unroll
-      for (int k = 1; k < N; ++k) cmac(s, a.e[i][k], conj(b.e[j][k]));
+      for (int n = 1; n < N; ++n) {
+        const int k = sum_term<N, T>(i, j, n);
+        cmac(s, a.e[i][k], conj(b.e[j][k]));
+      }
       c.e[i][j] = s;
     }
   return c;
@@ -248,9 +265,13 @@ template <int N, typename T> KLFT_HD Mat<N, T> mul_dd(const Mat<N, T> &a, const 
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<T> s = conj(a.e[0][i]) * conj(b.e[j][0]);
+      const int k0 = sum_term<N, T>(i, j, 0);
+      cx<T> s = conj(a.e[k0][i]) * conj(b.e[j][k0]);
 #pragma unroll
-      for (int k = 1; k < N; ++k) cmac(s, conj(a.e[k][i]), conj(b.e[j][k]));
+      for (int n = 1; n < N; ++n) {
+        const int k = sum_term<N, T>(i, j, n);
+        cmac(s, conj(a.e[k][i]), conj(b.e[j][k]));
+      }
       c.e[i][j] = s;
     }
   return c;
@@ -268,9 +289,13 @@ template <int N, typename T> KLFT_HD Mat<N, T> mul_dn(const Mat<N, T> &a, const 
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<T> s = conj(a.e[0][i]) * b.e[0][j];
+      const int k0 = sum_term<N, T>(i, j, 0);
+      cx<T> s = conj(a.e[k0][i]) * b.e[k0][j];
 #pragma unroll
-      for (int k = 1; k < N; ++k) cmac(s, conj(a.e[k][i]), b.e[k][j]);
+      for (int n = 1; n < N; ++n) {
+        const int k = sum_term<N, T>(i, j, n);
+        cmac(s, conj(a.e[k][i]), b.e[k][j]);
+      }
       c.e[i][j] = s;
     }
   return c;
@@ -302,9 +327,13 @@ template <int N, typename T> KLFT_HD T retr_mul(const Mat<N, T> &a, const Mat<N,
   T t = T(0);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    cx<T> s = a.e[i][0] * b.e[0][i];
+    const int k0 = sum_term<N, T>(i, i, 0);
+    cx<T> s = a.e[i][k0] * b.e[k0][i];
 #pragma unroll
-    for (int k = 1; k < N; ++k) cmac(s, a.e[i][k], b.e[k][i]);
+    for (int n = 1; n < N; ++n) {
+      const int k = sum_term<N, T>(i, i, n);
+      cmac(s, a.e[i][k], b.e[k][i]);
+    }
     t += s.re;
   }
   return t;
