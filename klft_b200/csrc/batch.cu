@@ -338,8 +338,8 @@ cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, i
 
 struct Group {
   GroupKey key;
-  long long sites = 0;  // of one pass, all chains
-  int lanes = 1;        // per site, or per link of the exp proposal
+  PassWork work;  // one pass, all chains
+  int lanes = 1;  // per site, or per link of the exp proposal
   std::vector<std::unique_ptr<ChainTable>> tables;
   std::vector<int> blocks;
 };
@@ -362,11 +362,11 @@ std::vector<Group> groups_of(const std::vector<klft::SweepItem> &items) {
       grp = &groups.back();
       grp->key = key;
     }
-    grp->sites += it.lat->g.Vh;
+    grp->work.add(it.lat->g, it.a);
   }
   for (auto &gg : groups)
-    gg.lanes = gg.key.exp ? exp_group_lanes(gg.key.dtype, gg.key.df, gg.sites << (gg.key.nd - 1))
-                          : group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.sites);
+    gg.lanes = gg.key.exp ? exp_group_lanes(gg.key.dtype, gg.key.df, gg.work.sites << (gg.key.nd - 1))
+                          : group_lanes(gg.key.nc, gg.key.dtype, gg.key.df, gg.work);
   return groups;
 }
 

@@ -775,7 +775,7 @@ static int sweep_block(klft_lattice *lat, const MetroArgs &a, const Defect &df, 
                          (lat->dtype() == 0 ? "_fp64" : "_mixed") +
                          (a.proposal == KLFT_PROPOSAL_EXP && lat->nc == 3 ? "_exp" : "_ref");
   const std::string key = tune_key(id, lat->g.nd, lat->g.H);
-  if (pass_lanes(lat->nc, lat->dtype(), a.proposal, df.active != 0, lat->g) > 1)
+  if (pass_lanes(lat->nc, lat->dtype(), a, df.active != 0, lat->g) > 1)
     return tuned_param(key, lat->g.nd, {128}, 128, [](int) { return 0.f; }, may_tune);
   auto time_fn = [&](int block) -> float {
     const size_t off = (lat->link_bytes + 255) & ~(size_t)255;

@@ -22,13 +22,27 @@ const double *bm_table();
 // (proposal 1), else the reference's 2^Nd site classes.
 KLFT_HD int metropolis_passes(int nc, int proposal, int nd) { return nc == 3 && proposal == 1 ? 2 * nd : 1 << nd; }
 
-// Reference proposals: lanes per site of a pass over `sites` sites (all chains of a
-// launch), 1 = one thread per site (site_update_ref), else metropolis_group.cuh.
-int group_lanes(int nc, int dtype, bool defect, long long sites);
+// One pass of a launch: its sites, and what its chains have in common.
+struct PassWork {
+  long long sites = 0;
+  int nd = 0, nhits_min = 0, nhits_max = 0;
+  double beta_min = 0.0;
+  void add(const Geom &g, const MetroArgs &a) {
+    const bool first = sites == 0;
+    sites += g.Vh;
+    nd = g.nd;
+    if (first || a.nhits < nhits_min) nhits_min = a.nhits;
+    if (first || a.nhits > nhits_max) nhits_max = a.nhits;
+    if (first || !(a.beta >= beta_min)) beta_min = a.beta;
+  }
+};
+// Reference proposals: lanes per site of a pass (all chains of a launch), 1 = one
+// thread per site (site_update_ref), else metropolis_group.cuh.
+int group_lanes(int nc, int dtype, bool defect, const PassWork &w);
 // The SU(3) exp proposal: lanes per link of a pass over `links` links.
 int exp_group_lanes(int dtype, bool defect, long long links);
-// What one of the two gives for a pass of one lattice (proposal as in MetroArgs).
-int pass_lanes(int nc, int dtype, int proposal, bool defect, const Geom &g);
+// What one of the two gives for a pass of one lattice.
+int pass_lanes(int nc, int dtype, const MetroArgs &a, bool defect, const Geom &g);
 constexpr int GROUP_THREADS = 64;  // per CTA of the group kernels: few sites over many SMs
 inline long long group_blocks(long long sites, int lanes) { return (sites * lanes + GROUP_THREADS - 1) / GROUP_THREADS; }
 

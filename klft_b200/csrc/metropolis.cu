@@ -8,6 +8,8 @@
 // of one thread per link (metropolis_site.cuh).  The per-site and per-link
 // updates are in metropolis_site.cuh.  Passes too small to fill the device so go
 // to groups of lanes (metropolis_group.cuh, metropolis_exp_group.cuh).
+#include <math.h>
+
 #include "metropolis_group.cuh"
 
 namespace klft {
@@ -98,19 +100,66 @@ static cudaError_t launch_nd(int nd, void *links, const Geom &g, int val, const 
 //               16: 255 309 392 776 1228 2759
 //   SU(2) FP32  1: 505 529 530 530 529 617     8: 180 192 194 283 543 1036
 //               16: 177 192 206 318 603 1514
-// and SU(3) at 256, 1200, 4096, 8192, 20736 (at the chain's own acceptance of 1 %; a
-// cold start, which accepts nothing, takes half as long):
-//   SU(3) FP64  1: 1611 1656 1685 1733 2232   32: 443 644 1627 3016 7295
-//                8: 706 764 989 1697 3883
-//   SU(3) FP32  1: 1486 1502 1517 1527 1855   32: 322 456 1038 1992 5099
-//                8: 536 572 781 1224 2402
-int group_lanes(int nc, int dtype, bool defect, long long sites) {
-  const bool f64 = dtype == 0;
-  if (nc == 3) return sites <= 1500 ? 32 : (sites <= (f64 ? 8200 : 12000) ? 8 : 1);
-  if (defect && !f64) return 1;  // no FP32 form for U(1), SU(2) with a defect
-  if (nc == 2) return f64 ? (sites <= 1000 ? 32 : (sites <= 5500 ? 16 : 1)) : (sites <= 7500 ? 8 : 1);
+// The hits enter where a site's places outgrow its window of the stream (U(1) FP32, at
+// 4 and 8 lanes over one thread: 7168 sites, nHits 13 0.44 0.49, 20 0.89 0.75, 30 1.19
+// 0.86, 60 1.51 1.05; 12,800 sites, nHits 20 1.06 1.18), and where few hits leave the
+// second wave of SU(2) FP64's CTAs (3552 sites fill the first) nothing to hide (16 lanes
+// over one thread at 4096 sites: nHits 1 1.44, 4 1.14, 10 0.91, 13 0.94, 30 1.05).
+static int group_lanes12(int nc, bool f64, const PassWork &w) {
+  const long long sites = w.sites;
+  const long long hits = (long long)w.nd * w.nhits_max;  // of a site
+  if (nc == 2 && f64) {
+    if (sites <= 1000) return 32;
+    return sites <= 3552 || (sites <= 5500 && w.nhits_min >= 8 && w.nhits_max <= 13) ? 16 : 1;
+  }
+  if (nc == 2) return sites <= 7500 ? 8 : 1;
   if (f64) return sites <= 1300 ? 32 : (sites <= 2500 ? 16 : (sites <= 9000 ? 8 : 1));
-  return sites <= 6000 ? 8 : (sites <= 16000 ? 4 : 1);
+  if (hits <= 60) return sites <= 6000 ? 8 : (sites <= 16000 ? 4 : 1);
+  return sites <= (hits <= 130 ? 9300 : 5500) ? 8 : 1;
+}
+
+// SU(3): a hit that lowers the action ends the chunk of proposals, so the groups win by
+// the rejected hits, and how many there are follows beta.  x = beta sqrt(2 (Nd - 1)), a
+// link's coupling to the sum of its staples when these are in no order, says where:
+// about 0.85 of the hits accepted at x = 1.2, 0.43 at 5, 0.23 at 7, 0.12 at 10, 0.05 at
+// 12, below 0.03 from 14 on.  us per sweep over one thread's, 4-D, nHits 10 (one thread:
+// FP64 1970-2010, 1700 at x = 14.7; FP32 1610-1650, 1500), equilibrium:
+//   sites  lanes   x = 1.2   4.9   7.3   9.8   12.2  14.0  14.7
+//   576    32 FP64    0.76  0.62  0.51  0.41  0.33  0.36  0.32   FP32 0.57 ..  0.22
+//   1152   32 FP64    0.94  0.73  0.60  0.48  0.39  0.44  0.40   FP32 0.86 ..  0.29
+//   1152   8  FP64    1.00  0.85  0.72  0.60  0.49  0.56  0.57   FP32 0.85 ..  0.42
+//   2304   8  FP64    1.01  0.87  0.75  0.62  0.51  0.58  0.60   FP32 0.86 ..  0.43
+//   4608   8  FP64    1.27  1.07  0.91  0.75  0.63  0.70  0.60
+//   4608   8  FP32    1.28  1.03  0.86  0.71  0.59  0.57  0.46
+//   6656   8  FP64    2.36  1.90  1.54  1.23  0.98  0.95  0.81
+//   6656   8  FP32    1.31  1.06  0.89  0.74  0.62  0.54  0.44
+//   8192   8  FP64    2.47  1.98  1.63  1.32  1.06  1.02  0.87
+//   8192   8  FP32    2.24  1.74  1.39  1.12  0.92  0.78  0.66
+// The steps are waves of CTAs: FP64 2368, 4736 sites at two and four CTAs per SM (592,
+// 1184 with 32 lanes), FP32 three and six (4736 in 2-D and 3-D).  Past the first full
+// wave one hit a link is too few (FP64 6656 sites, nHits 1: 1.10 at x = 14.7).
+static int group_lanes3(bool f64, const PassWork &w) {
+  const long long sites = w.sites;
+  const double x = w.beta_min * sqrt(2.0 * (w.nd - 1));
+  const bool second = w.nhits_min >= 8;  // enough hits for a second wave
+  if (f64) {
+    if (sites <= 592 || (sites <= 1184 && x >= 3.0) || (sites <= 1500 && x >= 12.0)) return 32;
+    const long long most = x >= 14.0 && second ? 8200 : (x >= 12.0 && second ? 6700 : (x >= 7.3 ? 4736 : (x >= 4.5 ? 2368 : 0)));
+    return sites <= most ? 8 : 1;
+  }
+  if (sites <= 1500) return 32;
+  const long long most = x >= 14.0 && second ? 12000
+                         : x >= 12.0 && second ? 8200
+                         : x >= 12.0 || (w.nd == 4 && x >= 7.0) ? 7104
+                         : x >= 7.0 ? 4736
+                         : x >= 4.5 ? 3552 : 2368;
+  return sites <= most ? 8 : 1;
+}
+
+int group_lanes(int nc, int dtype, bool defect, const PassWork &w) {
+  if (nc == 3) return group_lanes3(dtype == 0, w);
+  if (defect && dtype == 1) return 1;  // no FP32 form for U(1), SU(2) with a defect
+  return group_lanes12(nc, dtype == 0, w);
 }
 
 // The chain of a link's accepted products is repeated in every lane, so groups pay
@@ -125,16 +174,18 @@ int exp_group_lanes(int dtype, bool defect, long long links) {
   return links <= 2500 ? 16 : (links <= 6500 ? 4 : 1);
 }
 
-int pass_lanes(int nc, int dtype, int proposal, bool defect, const Geom &g) {
-  if (nc == 3 && proposal == PROPOSAL_EXP) return exp_group_lanes(dtype, defect, g.V / 2);
-  return group_lanes(nc, dtype, defect, g.Vh);
+int pass_lanes(int nc, int dtype, const MetroArgs &a, bool defect, const Geom &g) {
+  if (nc == 3 && a.proposal == PROPOSAL_EXP) return exp_group_lanes(dtype, defect, g.V / 2);
+  PassWork w;
+  w.add(g, a);
+  return group_lanes(nc, dtype, defect, w);
 }
 
 cudaError_t launch_metropolis_pass(int nc, int dtype, void *links, const Geom &g, int val, const MetroArgs &a,
                                    const uint32_t *d_sweep, unsigned long long *d_nacc, const Defect &df, int block,
                                    cudaStream_t st) {
   const bool exp = nc == 3 && a.proposal == PROPOSAL_EXP;
-  const int lanes = pass_lanes(nc, dtype, a.proposal, df.active != 0, g);
+  const int lanes = pass_lanes(nc, dtype, a, df.active != 0, g);
   if (lanes > 1) {
     MetroArgs b = a;
     // the FP64 exp(i eps H) proposal reads its Gaussians from the host-built table
