@@ -858,13 +858,19 @@ static cudaError_t wilson_gf_t(const void *links, const Geom &g, const int *cons
   char *up0 = base + al(es * Vc) + al(es * c[0].ncols);
   Links<N, T> U{(cx<T> *)links, g.V};
   if (!omega_ready) {
-    // Four segments while the columns alone leave the device waiting on their chains:
-    // one temporal 1x1 loop of SU(3) FP64 16^3x32 81 -> 61 us, 24^3x48 255 -> 212, 8^4
-    // FP32 32.7 -> 30.7; at 32^3 columns SU(3) 313 -> 312 FP64, 154.6 -> 156.7 FP32 (the
-    // second product of each row), U(1) 64 -> 61, SU(2) 84 -> 74.  Eight segments gave
+    // Four segments while the columns alone leave the device waiting on their chains.
+    // us of one temporal 1x1 loop with one segment and with four, by columns:
+    //   SU(3) FP64  4096 161 125   13,824 542 500   32,768 765 761   65,536 3636 3774
+    //   SU(3) FP32  4096  79  69   13,824 251 229   32,768 334 338   65,536 1731 1855
+    //   SU(2) FP64  4096  71  62   13,824 261 220   32,768 337 329   64,000  629  650
+    //   SU(2) FP32  4096  53  48   13,824 146 130   32,768 165 156   64,000  285  289
+    //   U(1)  FP64  4096  52  48   32,768 147 137   64,000 251 246   262,144  896  913
+    //   U(1)  FP32  4096  50  46   32,768 127 118   64,000 210 203   262,144  725  743
+    // (the second read of U_nu and the second product of each row).  Eight segments gave
     // no more.
     const long long ncols = c[0].ncols;
-    if (c[0].Lnu >= OMEGA_SEG && (N < 3 || ncols < 24000))
+    constexpr long long most = N == 1 ? 80000 : (N == 2 ? 48000 : 24000);
+    if (c[0].Lnu >= OMEGA_SEG && ncols < most)
       omega_seg_kernel<N, T, OMEGA_SEG><<<(unsigned)((ncols + 31) / 32), 32 * OMEGA_SEG, 0, st>>>(U, g, c[0], om, pol);
     else
       omega_kernel<N, T><<<(unsigned)((ncols + 127) / 128), 128, 0, st>>>(U, g, c[0], om, pol);
