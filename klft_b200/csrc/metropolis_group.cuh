@@ -187,119 +187,34 @@ KLFT_D int group_hits(const Mat<NC, T> &S, Mat<NC, T> &Uo, const MetroArgs &a, b
 }
 
 // ------------------------------------------------------------------ U(1), SU(2) in FP32
-// link_update_ref for a group, its products with their FMAs written out: the
-// compiler contracts a b + c d by the order in which it finds the operands, which
-// here is another one, and the FP32 chain is to be bit for bit the one of
-// site_update_ref (its accept decisions turn on the last bit).  Each form below is
-// the one that agrees with that function over 10^9 hits in 2, 3 and 4 dimensions.
-KLFT_D float mad2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }  // a b + c d
-
-template <int NC> struct Row0 { cx<float> v[NC]; };  // SU(2): row 0 of the matrix
-template <int NC> KLFT_D Row0<NC> row0(const Mat<NC, float> &m) {
-  Row0<NC> r;
-#pragma unroll
-  for (int j = 0; j < NC; ++j) r.v[j] = m.e[0][j];
-  return r;
-}
-// S U0
-KLFT_D Row0<1> group_mul_link(const Row0<1> &s, const Row0<1> &u) {
-  const cx<float> a = s.v[0], b = u.v[0];
-  return {{mk<float>(mad2(a.re, b.re, -a.im, b.im), mad2(a.im, b.re, a.re, b.im))}};
-}
-KLFT_D float su2_re00(const Row0<2> &x, const Row0<2> &y) {
-  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
-  return __fadd_rn(mad2(a.re, c.re, -a.im, c.im), mad2(b.re, -d.re, -b.im, d.im));
-}
-KLFT_D Row0<2> group_mul_link(const Row0<2> &s, const Row0<2> &u) {
-  const cx<float> a = s.v[0], b = s.v[1], c = u.v[0], d = u.v[1];
-  return {{mk<float>(su2_re00(s, u), __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.re, d.im, b.im, -d.re))),
-           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im)),
-                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
-}
-// A r
-KLFT_D Row0<1> group_mul_hit(const Row0<1> &x, const Row0<1> &r) { return group_mul_link(x, r); }
-KLFT_D Row0<2> group_mul_hit(const Row0<2> &x, const Row0<2> &r) {
-  const cx<float> a = x.v[0], b = x.v[1], c = r.v[0], d = r.v[1];
-  return {{mk<float>(su2_re00(x, r), __fadd_rn(mad2(a.re, c.im, a.im, c.re), mad2(b.re, d.im, b.im, -d.re))),
-           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.im, c.im, b.re, c.re)),
-                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
-}
-// Re Tr(Y M0)
-KLFT_D float group_retr(const Row0<1> &y, const Row0<1> &m) {
-  return mad2(y.v[0].re, m.v[0].re, -y.v[0].im, m.v[0].im);
-}
-KLFT_D float group_retr(const Row0<2> &y, const Row0<2> &m) {
-  const cx<float> a = y.v[0], b = y.v[1], c = m.v[0], d = m.v[1];
-  const float h = __fadd_rn(mad2(-a.im, c.im, a.re, c.re), mad2(b.re, -d.re, -b.im, d.im));
-  return __fadd_rn(h, h);
-}
-KLFT_D float group_retr(const Row0<1> &m) { return m.v[0].re; }
-KLFT_D float group_retr(const Row0<2> &m) { return __fadd_rn(m.v[0].re, m.v[0].re); }
-// restore(U0 A); FIRST: direction 0
-template <bool FIRST> KLFT_D Row0<1> group_new_link(const Row0<1> &u, const Row0<1> &x) {
-  const cx<float> a = u.v[0], c = x.v[0];
-  const float re = mad2(a.re, c.re, -a.im, c.im);
-  const float im = FIRST ? mad2(a.re, c.im, a.im, c.re) : mad2(a.im, c.re, a.re, c.im);
-  const float i = 1.0f / sqrtf(mad2(re, re, im, im));
-  return {{mk<float>(__fmul_rn(re, i), __fmul_rn(im, i))}};
-}
-template <bool FIRST> KLFT_D Row0<2> group_new_link(const Row0<2> &u, const Row0<2> &x) {
-  const cx<float> a = u.v[0], b = u.v[1], c = x.v[0], d = x.v[1];
-  cx<float> p, q;
-  p.re = su2_re00(u, x);
-  q.re = __fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im));
-  if constexpr (FIRST) {
-    p.im = __fadd_rn(mad2(a.re, c.im, a.im, c.re), mad2(b.re, d.im, b.im, -d.re));
-    q.im = __fadd_rn(mad2(a.re, d.im, a.im, d.re), mad2(b.re, -c.im, b.im, c.re));
-  } else {
-    p.im = __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.im, -d.re, b.re, d.im));
-    q.im = __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im));
-  }
-  const float i = 1.0f / sqrtf(fmaf(q.im, q.im, fmaf(q.re, q.re, mad2(p.re, p.re, p.im, p.im))));
-  return {{mk<float>(__fmul_rn(p.re, i), __fmul_rn(p.im, i)), mk<float>(__fmul_rn(q.re, i), __fmul_rn(q.im, i))}};
-}
-// Every lane runs the hits on the link and the staple as it loaded them, so lane 0
-// stores the new link between two barriers: no lane then reads it half way, and the
-// next direction's staple sees it.
+// The hits of link_update_f32 for a group.  Every lane runs them on the link and the
+// staple as it loaded them, so lane 0 stores the new link between two barriers: no lane
+// then reads it half way, and the next direction's staple sees it.
 template <int NC, int ND, int MU, typename Draws>
 KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &x, const MetroArgs &a, Draws &rng) {
   if constexpr (MU < ND) {
     if (open_link(g, x, MU)) return 0;
     const long long lx = site_lin(g, x);
-    const float bnc = (float)a.beta / (float)NC;
-    const Row0<NC> S = row0(staple_ct<NC, ND, MU, float>(U, g, x)), U0 = row0(U.load(lx, MU));
-    const Row0<NC> M0 = group_mul_link(S, U0);
-    Row0<NC> A = row0(mident<NC, float>());
-    float trO = group_retr(M0);
-    int nacc = 0;
+    Hits32<NC> h(row0(staple_ct<NC, ND, MU, float>(U, g, x)), row0(U.load(lx, MU)), (float)a.beta / (float)NC);
 #pragma unroll 1
     for (int hit = 0; hit < a.nhits;) {
       const int m = rng.ready(a.nhits - hit);
       hit += m;
 #pragma unroll 1
       for (int k = 0; k < m; ++k) {
-        const Row0<NC> Y = group_mul_hit(A, row0(rng.propose_next()));
-        const float tY = group_retr(Y, M0);
-        const float dS = __fmul_rn(-bnc, __fsub_rn(tY, trO));
+        const float dS = h.propose(row0(rng.propose_next()));
         const bool accept = rng.accept(dS);  // ln u <= 0: also of dS < 0
         rng.advance(!(dS < 0.f));
-        if (accept) {
-          A = Y;
-          trO = tY;
-          ++nacc;
-        }
+        if (accept) h.accept();
       }
     }
-    if (nacc) {
-      const Row0<NC> V = group_new_link<MU == 0>(U0, A);
-      Mat<NC, float> m;
-#pragma unroll
-      for (int j = 0; j < NC; ++j) m.e[0][j] = V.v[j];
+    if (h.nacc) {
+      const Mat<NC, float> m = h.template link<MU == 0>();
       __syncwarp(rng.mask);
       if (rng.gl == 0) U.store(lx, MU, m);
       __syncwarp(rng.mask);
     }
-    return nacc;
+    return h.nacc;
   }
   return 0;
 }
