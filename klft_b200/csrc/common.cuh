@@ -54,7 +54,13 @@ KLFT_HD double u53(uint32_t hi, uint32_t lo) {
   return (double)((((uint64_t)hi << 32) | lo) >> 11) * 0x1.0p-53;
 }
 // Kokkos drand(start, end) = start + (end - start) * u
-KLFT_HD double drand_u(double a, double b, double u) { return a + (b - a) * u; }
+KLFT_HD double drand_u(double a, double b, double u) {
+#ifdef __CUDA_ARCH__
+  return fma(b - a, u, a);  // as the compiler contracts it
+#else
+  return a + (b - a) * u;
+#endif
+}
 
 // Sequential stream of 53-bit uniforms in [0,1).  key = (lo32(seed),
 // hi32(seed) ^ lo32(chain)), counter = (block, site, step, kind<<24 | sub).

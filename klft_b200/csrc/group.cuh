@@ -13,7 +13,7 @@ constexpr double K2PI = 6.283185307179586;
 enum Proposal : int { PROPOSAL_REFERENCE = 0, PROPOSAL_EXP = 1 };
 
 // ------------------------------------------------------------------ proposals
-// The proposals read NPROP<NC> consecutive uniforms of the site's stream (SU(3):
+// The proposals read RefDraws<NC>::n consecutive uniforms of the site's stream (SU(3):
 // 12 unless a drawn vector has norm zero); the accept uniform, when drawn, follows.
 template <int NC> struct RefDraws { static constexpr int n = NC == 1 ? 1 : (NC == 2 ? 3 : 12); };
 
@@ -30,7 +30,7 @@ template <typename T> KLFT_D Mat<2, T> propose(const double *w, double delta, co
   const T u = (T)drand_u(-1.0, 1.0, w[1]);
   const T theta = (T)drand_u(0.0, 2.0 * KPI, w[2]);
   const T salpha = sin(alpha);
-  const T su = sqrt(T(1) - u * u);
+  const T su = sqrt(fma(-u, u, T(1)));
   const T n1 = su * sin(theta);
   const T n2 = su * cos(theta);
   Mat<2, T> r;

@@ -195,7 +195,7 @@ KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &
   if constexpr (MU < ND) {
     if (open_link(g, x, MU)) return 0;
     const long long lx = site_lin(g, x);
-    Hits32<NC> h(row0(staple_ct<NC, ND, MU, float>(U, g, x)), row0(U.load(lx, MU)), (float)a.beta / (float)NC);
+    Hits32<NC> h(staple_f32<NC, ND, MU>(U, g, x), row0(U.load(lx, MU)), (float)a.beta / (float)NC);
 #pragma unroll 1
     for (int hit = 0; hit < a.nhits;) {
       const int m = rng.ready(a.nhits - hit);

@@ -165,33 +165,9 @@ template <int NC> struct HitDraws {
 // which differs from kernel to kernel, and an accept decision turns on the last bit.  So
 // a chain is the same bit for bit whichever kernel its lattice's size, or the size of its
 // batch, selects.  The forms are the ones nvcc 12.9 chose for this update, found by
-// comparing chains over 10^9 hits in 2, 3 and 4 dimensions.
-KLFT_D float mad2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }  // a b + c d
-
-template <int NC> struct Row0 { cx<float> v[NC]; };  // SU(2): row 0 of the matrix
-template <int NC> KLFT_D Row0<NC> row0(const Mat<NC, float> &m) {
-  Row0<NC> r;
-#pragma unroll
-  for (int j = 0; j < NC; ++j) r.v[j] = m.e[0][j];
-  return r;
-}
-// S U0
-KLFT_D Row0<1> f32_mul_link(const Row0<1> &s, const Row0<1> &u) {
-  const cx<float> a = s.v[0], b = u.v[0];
-  return {{mk<float>(mad2(a.re, b.re, -a.im, b.im), mad2(a.im, b.re, a.re, b.im))}};
-}
-KLFT_D float su2_re00(const Row0<2> &x, const Row0<2> &y) {
-  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
-  return __fadd_rn(mad2(a.re, c.re, -a.im, c.im), mad2(b.re, -d.re, -b.im, d.im));
-}
-KLFT_D Row0<2> f32_mul_link(const Row0<2> &s, const Row0<2> &u) {
-  const cx<float> a = s.v[0], b = s.v[1], c = u.v[0], d = u.v[1];
-  return {{mk<float>(su2_re00(s, u), __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.re, d.im, b.im, -d.re))),
-           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im)),
-                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
-}
+// comparing chains over 10^9 hits in 2, 3 and 4 dimensions.  Staples: staple_f32.
 // A r
-KLFT_D Row0<1> f32_mul_hit(const Row0<1> &x, const Row0<1> &r) { return f32_mul_link(x, r); }
+KLFT_D Row0<1> f32_mul_hit(const Row0<1> &x, const Row0<1> &r) { return f32_mul(x, r); }
 KLFT_D Row0<2> f32_mul_hit(const Row0<2> &x, const Row0<2> &r) {
   const cx<float> a = x.v[0], b = x.v[1], c = r.v[0], d = r.v[1];
   return {{mk<float>(su2_re00(x, r), __fadd_rn(mad2(a.re, c.im, a.im, c.re), mad2(b.re, d.im, b.im, -d.re))),
@@ -239,7 +215,7 @@ template <int NC> struct Hits32 {
   float trO, tY, bnc;
   int nacc = 0;
   KLFT_D Hits32(const Row0<NC> &S, const Row0<NC> &U, float bnc_)
-      : U0(U), M0(f32_mul_link(S, U)), A(row0(mident<NC, float>())), trO(f32_retr(M0)), bnc(bnc_) {}
+      : U0(U), M0(f32_mul(S, U)), A(row0(mident<NC, float>())), trO(f32_retr(M0)), bnc(bnc_) {}
   KLFT_D float propose(const Row0<NC> &r) {
     Y = f32_mul_hit(A, r);
     tY = f32_retr(Y, M0);
@@ -263,7 +239,7 @@ template <int NC> struct Hits32 {
 template <int NC, int ND, int MU, typename Draws>
 KLFT_D int link_update_f32(const Links<NC, float> &U, const Geom &g, const Site &x, const MetroArgs &a, Draws &rng,
                            long long lx, float bnc) {
-  Hits32<NC> h(row0(staple_ct<NC, ND, MU, float>(U, g, x)), row0(U.load(lx, MU)), bnc);
+  Hits32<NC> h(staple_f32<NC, ND, MU>(U, g, x), row0(U.load(lx, MU)), bnc);
 #pragma unroll 1
   for (int hit = 0; hit < a.nhits; ++hit) {
     double u;

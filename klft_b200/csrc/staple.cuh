@@ -160,6 +160,83 @@ KLFT_D Mat<NC, T> staple_ct(const Links<NC, T> &U, const Geom &g, const Site &x,
   return S;
 }
 
+// ------------------------------------------------------------------ U(1), SU(2) in FP32
+// Products with their FMAs written out, on what is stored of a link: row 0, of which an
+// SU(2) element's row 1 is (-conj(v1), conj(v0)).
+KLFT_D float mad2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }  // a b + c d
+
+template <int NC> struct Row0 { cx<float> v[NC]; };  // SU(2): row 0 of the matrix
+template <int NC> KLFT_D Row0<NC> row0(const Mat<NC, float> &m) {
+  Row0<NC> r;
+#pragma unroll
+  for (int j = 0; j < NC; ++j) r.v[j] = m.e[0][j];
+  return r;
+}
+// a b
+KLFT_D Row0<1> f32_mul(const Row0<1> &x, const Row0<1> &y) {
+  const cx<float> a = x.v[0], b = y.v[0];
+  return {{mk<float>(mad2(a.re, b.re, -a.im, b.im), mad2(a.im, b.re, a.re, b.im))}};
+}
+KLFT_D float su2_re00(const Row0<2> &x, const Row0<2> &y) {
+  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
+  return __fadd_rn(mad2(a.re, c.re, -a.im, c.im), mad2(b.re, -d.re, -b.im, d.im));
+}
+KLFT_D Row0<2> f32_mul(const Row0<2> &x, const Row0<2> &y) {
+  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
+  return {{mk<float>(su2_re00(x, y), __fadd_rn(mad2(a.im, c.re, a.re, c.im), mad2(b.re, d.im, b.im, -d.re))),
+           mk<float>(__fadd_rn(mad2(a.re, d.re, -a.im, d.im), mad2(b.re, c.re, b.im, c.im)),
+                     __fadd_rn(mad2(a.im, d.re, a.re, d.im), mad2(b.im, c.re, b.re, -c.im)))}};
+}
+// a b^+
+KLFT_D Row0<1> f32_mul_nd(const Row0<1> &x, const Row0<1> &y) {
+  const cx<float> a = x.v[0], b = y.v[0];
+  return {{mk<float>(mad2(a.re, b.re, a.im, b.im), mad2(a.im, b.re, a.re, -b.im))}};
+}
+KLFT_D Row0<2> f32_mul_nd(const Row0<2> &x, const Row0<2> &y) {
+  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
+  return {{mk<float>(__fadd_rn(mad2(a.re, c.re, a.im, c.im), mad2(b.re, d.re, b.im, d.im)),
+                     __fadd_rn(mad2(a.im, c.re, a.re, -c.im), mad2(b.im, d.re, b.re, -d.im))),
+           mk<float>(__fadd_rn(mad2(a.im, d.im, a.re, -d.re), mad2(b.re, c.re, -b.im, c.im)),
+                     __fadd_rn(mad2(a.im, -d.re, a.re, -d.im), mad2(b.im, c.re, b.re, c.im)))}};
+}
+// a^+ b^+
+KLFT_D Row0<1> f32_mul_dd(const Row0<1> &x, const Row0<1> &y) {
+  const cx<float> a = x.v[0], b = y.v[0];
+  return {{mk<float>(mad2(a.re, b.re, a.im, -b.im), mad2(-a.im, b.re, a.re, -b.im))}};
+}
+KLFT_D Row0<2> f32_mul_dd(const Row0<2> &x, const Row0<2> &y) {
+  const cx<float> a = x.v[0], b = x.v[1], c = y.v[0], d = y.v[1];
+  return {{mk<float>(__fadd_rn(mad2(a.re, c.re, a.im, -c.im), mad2(-b.re, d.re, b.im, -d.im)),
+                     __fadd_rn(mad2(-a.im, c.re, a.re, -c.im), mad2(b.re, d.im, -b.im, d.re))),
+           mk<float>(__fadd_rn(mad2(a.re, -d.re, a.im, -d.im), mad2(b.im, c.im, -b.re, c.re)),
+                     __fadd_rn(mad2(-a.im, -d.re, a.re, -d.im), mad2(-b.im, c.re, -b.re, c.im)))}};
+}
+template <int NC> KLFT_D void f32_add(Row0<NC> &s, const Row0<NC> &a) {
+#pragma unroll
+  for (int j = 0; j < NC; ++j) s.v[j] = mk<float>(__fadd_rn(s.v[j].re, a.v[j].re), __fadd_rn(s.v[j].im, a.v[j].im));
+}
+// The staple of U_mu(x), mu = MU, without a defect: the terms of staple_ct.  The forms
+// are those nvcc 12.9 chose for staple_ct in the Metropolis passes, the same in every
+// direction and dimension: found one product and component at a time on fields whose
+// other terms cancel exactly, so that the sum left is zero or a rounding error.
+template <int NC, int ND, int MU> KLFT_D Row0<NC> staple_f32(const Links<NC, float> &U, const Geom &g, const Site &x) {
+  auto link = [&](const Site &s, int mu) { return row0(U.load(site_lin(g, s), mu)); };
+  Row0<NC> S = row0(mzero<NC, float>());
+  const Site xpmu = site_up(g, x, MU);
+#pragma unroll
+  for (int nu = 0; nu < ND; ++nu) {
+    if (nu == MU) continue;
+    f32_add(S, f32_mul_nd(f32_mul_nd(link(xpmu, nu), link(site_up(g, x, nu), MU)), link(x, nu)));
+  }
+#pragma unroll
+  for (int nu = 0; nu < ND; ++nu) {
+    if (nu == MU) continue;
+    const Site xmnu = site_dn(g, x, nu);
+    f32_add(S, f32_mul(f32_mul_dd(link(site_dn(g, xpmu, nu), nu), link(xmnu, MU)), link(xmnu, nu)));
+  }
+  return S;
+}
+
 // staple_ct for a run-time mu (uniform across a warp in the callers)
 template <int NC, int ND, typename T>
 KLFT_D Mat<NC, T> staple_dispatch(const Links<NC, T> &U, const Geom &g, const Site &x, int mu) {
