@@ -100,11 +100,16 @@ static cudaError_t launch_nd(int nd, void *links, const Geom &g, int val, const 
 //               16: 255 309 392 776 1228 2759
 //   SU(2) FP32  1: 505 529 530 530 529 617     8: 180 192 194 283 543 1036
 //               16: 177 192 206 318 603 1514
-// The hits enter where a site's places outgrow its window of the stream (U(1) FP32, at
-// 4 and 8 lanes over one thread: 7168 sites, nHits 13 0.44 0.49, 20 0.89 0.75, 30 1.19
-// 0.86, 60 1.51 1.05; 12,800 sites, nHits 20 1.06 1.18), and where few hits leave the
-// second wave of SU(2) FP64's CTAs (3552 sites fill the first) nothing to hide (16 lanes
-// over one thread at 4096 sites: nHits 1 1.44, 4 1.14, 10 0.91, 13 0.94, 30 1.05).
+// The hits of a site enter where their places outgrow its window of the stream, and where
+// few of them leave the second wave of SU(2) FP64's CTAs nothing to hide.  us per sweep
+// over one thread's, 4-D, by nHits:
+//   U(1) FP32   7168 sites   13: 0.44 (4 lanes) 0.49 (8)   20: 0.89 0.75   30: 1.19 0.86   60: 1.51 1.05
+//              12,800 sites  13: 0.59 0.83   20: 1.06 1.18
+//   U(1) FP64   4608 sites   20: 0.59 (16) 0.61 (8)   60: 0.69 0.85   300: 0.70 0.85
+//               7168 sites   20: 0.99 0.74   60: 1.07 1.04   300: 1.08 1.08
+//   SU(2) FP32  3136 sites   30: 0.84 (8)   60: 0.95   300: 1.02;   4608 sites  0.97 1.09 1.20
+//   SU(2) FP64  4096 sites    1: 1.44 (16)   4: 1.14   10: 0.91   13: 0.94   30: 1.04
+// Waves: 3552 sites of SU(2) FP64 with 16 lanes, 7104 of SU(2) FP32 with 8.
 static int group_lanes12(int nc, bool f64, const PassWork &w) {
   const long long sites = w.sites;
   const long long hits = (long long)w.nd * w.nhits_max;  // of a site
@@ -112,8 +117,12 @@ static int group_lanes12(int nc, bool f64, const PassWork &w) {
     if (sites <= 1000) return 32;
     return sites <= 3552 || (sites <= 5500 && w.nhits_min >= 8 && w.nhits_max <= 13) ? 16 : 1;
   }
-  if (nc == 2) return sites <= 7500 ? 8 : 1;
-  if (f64) return sites <= 1300 ? 32 : (sites <= 2500 ? 16 : (sites <= 9000 ? 8 : 1));
+  if (nc == 2) return sites <= (hits <= 150 ? 7104 : 3200) ? 8 : 1;
+  if (f64) {
+    if (sites <= 1300) return 32;
+    if (hits > 130) return sites <= 5900 ? 16 : 1;
+    return sites <= 2500 ? 16 : (sites <= 9000 ? 8 : 1);
+  }
   if (hits <= 60) return sites <= 6000 ? 8 : (sites <= 16000 ? 4 : 1);
   return sites <= (hits <= 130 ? 9300 : 5500) ? 8 : 1;
 }
@@ -147,7 +156,7 @@ static int group_lanes3(bool f64, const PassWork &w) {
     const long long most = x >= 14.0 && second ? 8200 : (x >= 12.0 && second ? 6700 : (x >= 7.3 ? 4736 : (x >= 4.5 ? 2368 : 0)));
     return sites <= most ? 8 : 1;
   }
-  if (sites <= 1500) return 32;
+  if (sites <= 1184 || (sites <= 1500 && x >= 3.0)) return 32;
   const long long most = x >= 14.0 && second ? 12000
                          : x >= 12.0 && second ? 8200
                          : x >= 12.0 || (w.nd == 4 && x >= 7.0) ? 7104
