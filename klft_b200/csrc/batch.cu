@@ -269,7 +269,7 @@ struct GroupKey {
 };
 
 template <int NC, int ND, typename T, bool EXP, bool DF>
-cudaError_t launch_group_t(const ChainTable &tab, int blocks, int val, unsigned long long *nacc, const uint32_t *slot,
+cudaError_t launch_multi_t(const ChainTable &tab, int blocks, int val, unsigned long long *nacc, const uint32_t *slot,
                            cudaStream_t st) {
   if constexpr (EXP && NC == 3) {
     // one kernel instance per link direction (compiled staple site steps)
@@ -292,22 +292,22 @@ cudaError_t launch_group_t(const ChainTable &tab, int blocks, int val, unsigned 
 }
 
 template <int NC, int ND, typename T>
-cudaError_t launch_group_nd(const GroupKey &k, const ChainTable &tab, int blocks, int val, unsigned long long *nacc,
+cudaError_t launch_multi_nd(const GroupKey &k, const ChainTable &tab, int blocks, int val, unsigned long long *nacc,
                             const uint32_t *slot, cudaStream_t st) {
   if (k.exp) {
-    if (k.df) return launch_group_t<NC, ND, T, true, true>(tab, blocks, val, nacc, slot, st);
-    return launch_group_t<NC, ND, T, true, false>(tab, blocks, val, nacc, slot, st);
+    if (k.df) return launch_multi_t<NC, ND, T, true, true>(tab, blocks, val, nacc, slot, st);
+    return launch_multi_t<NC, ND, T, true, false>(tab, blocks, val, nacc, slot, st);
   }
-  if (k.df) return launch_group_t<NC, ND, T, false, true>(tab, blocks, val, nacc, slot, st);
-  return launch_group_t<NC, ND, T, false, false>(tab, blocks, val, nacc, slot, st);
+  if (k.df) return launch_multi_t<NC, ND, T, false, true>(tab, blocks, val, nacc, slot, st);
+  return launch_multi_t<NC, ND, T, false, false>(tab, blocks, val, nacc, slot, st);
 }
 
 template <int NC, typename T>
-cudaError_t launch_group_nc(const GroupKey &k, const ChainTable &tab, int blocks, int val, unsigned long long *nacc,
+cudaError_t launch_multi_nc(const GroupKey &k, const ChainTable &tab, int blocks, int val, unsigned long long *nacc,
                             const uint32_t *slot, cudaStream_t st) {
-  if (k.nd == 2) return launch_group_nd<NC, 2, T>(k, tab, blocks, val, nacc, slot, st);
-  if (k.nd == 3) return launch_group_nd<NC, 3, T>(k, tab, blocks, val, nacc, slot, st);
-  return launch_group_nd<NC, 4, T>(k, tab, blocks, val, nacc, slot, st);
+  if (k.nd == 2) return launch_multi_nd<NC, 2, T>(k, tab, blocks, val, nacc, slot, st);
+  if (k.nd == 3) return launch_multi_nd<NC, 3, T>(k, tab, blocks, val, nacc, slot, st);
+  return launch_multi_nd<NC, 4, T>(k, tab, blocks, val, nacc, slot, st);
 }
 
 // lanes > 1: the pass by groups of lanes (metropolis_group.cuh, metropolis_exp_group.cuh)
@@ -327,13 +327,13 @@ cudaError_t launch_group(const GroupKey &k, const ChainTable &tab, int blocks, i
     return launch_group_su3(k.nd, k.dtype, lanes, k.df, l);
   }
   if (k.dtype == 0) {
-    if (k.nc == 1) return launch_group_nc<1, double>(k, tab, blocks, val, nacc, slot, st);
-    if (k.nc == 2) return launch_group_nc<2, double>(k, tab, blocks, val, nacc, slot, st);
-    return launch_group_nc<3, double>(k, tab, blocks, val, nacc, slot, st);
+    if (k.nc == 1) return launch_multi_nc<1, double>(k, tab, blocks, val, nacc, slot, st);
+    if (k.nc == 2) return launch_multi_nc<2, double>(k, tab, blocks, val, nacc, slot, st);
+    return launch_multi_nc<3, double>(k, tab, blocks, val, nacc, slot, st);
   }
-  if (k.nc == 1) return launch_group_nc<1, float>(k, tab, blocks, val, nacc, slot, st);
-  if (k.nc == 2) return launch_group_nc<2, float>(k, tab, blocks, val, nacc, slot, st);
-  return launch_group_nc<3, float>(k, tab, blocks, val, nacc, slot, st);
+  if (k.nc == 1) return launch_multi_nc<1, float>(k, tab, blocks, val, nacc, slot, st);
+  if (k.nc == 2) return launch_multi_nc<2, float>(k, tab, blocks, val, nacc, slot, st);
+  return launch_multi_nc<3, float>(k, tab, blocks, val, nacc, slot, st);
 }
 
 struct Group {

@@ -10,9 +10,10 @@
 //
 //  * U(1), SU(2): the lanes form the uniforms of a window of the stream and the
 //    proposal that would start at each place in it; a hit then takes the one at
-//    its place.  Most are not used (a hit moves on by 1-2 or 3-4 places).  The
-//    links around the site are brought into L1 by all lanes at once, then every
-//    lane runs link_update_ref.
+//    its place.  Most are not used (a hit moves on by 1-2 or 3-4 places).  In
+//    FP64 the staples' products are shared out as for SU(3) (group_hits); in FP32
+//    the links around the site are brought into L1 by all lanes at once, then
+//    every lane forms the staples (group_link_f32).  Every lane runs the hits.
 //  * SU(3), where a few per cent of the hits are accepted: lane j forms the
 //    proposal and the action change of the j-th hit from here, as if every hit
 //    before it were rejected with its uniform drawn; the group keeps the hits
@@ -156,13 +157,13 @@ KLFT_D void touch_neighbours(const Links<NC, T> &U, const Geom &g, const Site &x
 // ------------------------------------------------------------------ U(1), SU(2) in FP64
 // The hits of a link with staple S, as in link_update_ref; Uo: the link, updated when
 // any is accepted.
-template <int NC, typename T, typename Draws>
-KLFT_D int group_hits(const Mat<NC, T> &S, Mat<NC, T> &Uo, const MetroArgs &a, bool dlink, const Defect &df,
-                      Draws &rng, T bnc) {
-  const Mat<NC, T> U0 = Uo, M0 = mul(S, U0);
-  const T cdef = dlink ? (T)defect_c(df) : T(1);
-  Mat<NC, T> A = mident<NC, T>();
-  T trO = retr_diag(M0);
+template <int NC, typename Draws>
+KLFT_D int group_hits(const Mat<NC, double> &S, Mat<NC, double> &Uo, const MetroArgs &a, bool dlink, const Defect &df,
+                      Draws &rng, double bnc) {
+  const Mat<NC, double> U0 = Uo, M0 = mul(S, U0);
+  const double cdef = dlink ? defect_c(df) : 1.0;
+  Mat<NC, double> A = mident<NC, double>();
+  double trO = retr_diag(M0);
   int nacc = 0;
 #pragma unroll 1
   for (int hit = 0; hit < a.nhits;) {
@@ -170,11 +171,11 @@ KLFT_D int group_hits(const Mat<NC, T> &S, Mat<NC, T> &Uo, const MetroArgs &a, b
     hit += m;
 #pragma unroll 1
     for (int k = 0; k < m; ++k) {
-      const Mat<NC, T> Y = mul(A, rng.propose_next());
-      const T tY = retr_mul(Y, M0);
-      const T dS = -bnc * (tY - trO) * cdef;
+      const Mat<NC, double> Y = mul(A, rng.propose_next());
+      const double tY = retr_mul(Y, M0);
+      const double dS = -bnc * (tY - trO) * cdef;
       const bool accept = rng.accept(dS);  // ln u <= 0: also of dS < 0
-      rng.advance(!(dS < T(0)));
+      rng.advance(!(dS < 0.0));
       if (accept) {
         A = Y;
         trO = tY;
@@ -387,8 +388,8 @@ template <typename T, int G> struct LaneHits3 {
 
 // ------------------------------------------------------------------ one site
 // Whether the staples are formed from shared parts.  In FP32 U(1) and SU(2) they
-// are not: their sums of two products are contracted by context too, so every lane
-// forms the staple as site_update_ref does, from links already in L1.
+// are not: every lane forms the staple as site_update_ref does (staple_f32), from
+// links already in L1.
 template <int NC, typename T> struct SharedStaples { static constexpr bool v = NC == 3 || sizeof(T) == 8; };
 
 template <int NC, int ND, typename T, int G> struct GroupShared {
@@ -428,7 +429,7 @@ KLFT_D int group_site_update(GroupShared<NC, ND, T, G> *shared, const Links<NC, 
     if (ok) {
       if constexpr (SharedStaples<NC, T>::v) {
         n = group_links<NC, ND, T, DF, G>(sh.parts, U, g, x, df, [&](const Mat<NC, T> &S, Mat<NC, T> &V, bool dlink) {
-          return group_hits<NC, T>(S, V, a, dlink, df, rng, bnc);
+          return group_hits<NC>(S, V, a, dlink, df, rng, bnc);
         });
       } else {
         // every lane: the same links and decisions
