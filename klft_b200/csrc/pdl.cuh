@@ -16,7 +16,8 @@ namespace klft {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// dependent: the operation before in the stream is a kernel (else an ordinary launch)
+// dependent: the operation before in the stream is a kernel (else an ordinary launch).
+// A launch that is refused does not leave its error behind for the next call to report.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_after(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                          Args &&...args) {
@@ -30,7 +31,9 @@ cudaError_t launch_after(bool dependent, void (*kernel)(KArgs...), dim3 grid, di
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
 }
 
 }  // namespace klft
