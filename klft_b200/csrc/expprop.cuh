@@ -50,7 +50,8 @@ template <typename V> struct XMat { V re[3][3], im[3][3]; };
 // (d c0, a + d c1, b), and exp(iQ) = f0 + f1 Q + f2 Q^2 with
 // f = sum_n i^n / n! (a_n, b_n, d_n).  Arguments with c1 > 3/4 (an eigenvalue
 // possibly above 1: |lambda|^2 <= 4 c1 / 3) are scaled by 2^-k and the result
-// squared k times in coefficient space:
+// squared k times in coefficient space, all in the basis of the scaled Q (c0, c1
+// its own):
 //   (f0 + f1 Q + f2 Q^2)^2 = (f0^2 + 2 f1 f2 c0) + (2 f0 f1 + 2 f1 f2 c1 + f2^2 c0) Q
 //                          + (f1^2 + 2 f0 f2 + f2^2 c1) Q^2.
 template <typename V> KLFT_D XMat<V> expi_gellmann(const V h[8], V s) {
@@ -122,8 +123,6 @@ template <typename V> KLFT_D XMat<V> expi_gellmann(const V h[8], V s) {
     const V g2i = vfma(f22i, cs1, vfma(splat<V>(2.0), vfma(f0r, f2i, vmul(f0i, f2r)),
                                        vmul(splat<V>(2.0), vmul(f1r, f1i))));
     f0r = g0r; f0i = g0i; f1r = g1r; f1i = g1i; f2r = g2r; f2i = g2i;
-    cs1 = vmul(cs1, splat<V>(4.0));
-    cs0 = vmul(cs0, splat<V>(8.0));
   }
   // back to the basis (1, Q, Q^2): Q' = scale Q
   if (sq) {
