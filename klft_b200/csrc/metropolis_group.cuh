@@ -19,8 +19,8 @@
 //    before it were rejected with its uniform drawn; the group keeps the hits
 //    before the first exception, applies that one and goes on from there.  The
 //    products of neighbour links in the staples of all directions are shared out
-//    as well: links of one class are not neighbours, so only U_nu(x) itself
-//    changes while the site is updated.
+//    as well (StapleParts in FP64, StapleTerms in FP32): links of one class are
+//    not neighbours, so only U_nu(x) itself changes while the site is updated.
 //
 // None of the proposals read links, so the first ones come before the wait for
 // the pass before (programmatic dependent launch).  Operations on a link and
@@ -221,16 +221,8 @@ KLFT_D int group_link_f32(const Links<NC, float> &U, const Geom &g, const Site &
 }
 
 // ------------------------------------------------------------------ staples shared out
-// m as Links::load returns it after Links::store(m)
-template <int NC, typename T> KLFT_D Mat<NC, T> as_stored(Mat<NC, T> m) {
-  if constexpr (LinkPlanes<NC, T>::n < NC * NC) {
-    if constexpr (NC == 3) complete_row2(m);
-    else su2_row1(m);
-  }
-  return m;
-}
-
-// The links of a site and the products of its neighbours' links, per group.
+// FP64 (every element of a link is stored): the links of a site and the products of its
+// neighbours' links, per group.
 template <int NC, int ND, typename T> struct StapleParts {
   Mat<NC, T> own[ND];
   // [mu][forward nu, backward nu]: U_nu(x+mu) U_mu(x+nu)^+, the whole backward term
@@ -274,9 +266,99 @@ template <int NC, int ND, typename T> struct StapleParts {
   }
 };
 
-// The links of site x in the order mu = 0 .. Nd-1 from shared parts; hits(S, U, dlink)
-// updates one link and returns its accepted hits, the same in every lane.
-template <int NC, int ND, typename T, bool DF, int G, typename Hits>
+// SU(3) in FP32: the same products, each formed as staple() forms it, so that the
+// compiler contracts them as it does there (StapleParts gave other last bits: one accept
+// decision in 10^7 on disordered links).  The last product of a forward term, which
+// reads a link of the site, is one lane's.  With a defect the form of the shared
+// products differed once more, so there each lane forms a whole term of one link's
+// staple.  us per sweep at nHits 10, beta = 6, without a defect 8^4 210, 16^4 549; with
+// whole terms 298, 594; one thread per site 1500 in both.
+template <int ND> struct StapleTerms {
+  static constexpr int NT = 2 * (ND - 1);  // terms of a link: forward nu, then backward nu
+  Mat<3, float> part[ND * NT];             // [mu][term]; with a defect the terms of one link
+  Mat<3, float> fwd[ND - 1];
+
+  // first product of forward term r, or all of backward term r
+  template <bool DF>
+  static KLFT_D Mat<3, float> product(const Links<3, float> &U, const Geom &g, const Site &x, int mu, int r, int nu,
+                                      const Defect &df) {
+    const Site xpmu = site_up(g, x, mu);
+    if (r < ND - 1)
+      return mul_nd(load_link<3, float, DF>(U, g, xpmu, nu, df),
+                    load_link<3, float, DF>(U, g, site_up(g, x, nu), mu, df));
+    const Site xmnu = site_dn(g, x, nu);
+    const Mat<3, float> t = mul_dd(load_link<3, float, DF>(U, g, site_dn(g, xpmu, nu), nu, df),
+                                   load_link<3, float, DF>(U, g, xmnu, mu, df));
+    return mul(t, load_link<3, float, DF>(U, g, xmnu, nu, df));
+  }
+  static KLFT_D int nu_of(int mu, int r) {
+    const int nu = r < ND - 1 ? r : r - (ND - 1);
+    return nu + (nu >= mu);
+  }
+
+  template <bool DF, int G>
+  KLFT_D void load(const Links<3, float> &U, const Geom &g, const Site &x, const Defect &df, int gl) {
+    if constexpr (DF) touch_neighbours<3, ND, float, G>(U, g, x, gl);
+    else
+      for (int q = gl; q < ND * NT; q += G) {
+        const int mu = q / NT, r = q - mu * NT;
+        part[q] = product<DF>(U, g, x, mu, r, nu_of(mu, r), df);
+      }
+  }
+
+  template <bool DF, int G>
+  KLFT_D Mat<3, float> staple(const Links<3, float> &U, const Geom &g, const Site &x, int mu, const Defect &df, int gl,
+                              unsigned mask) {
+    const Mat<3, float> *p = part;
+    if constexpr (DF) {
+      for (int r = gl; r < NT; r += G) {
+        const int nu = nu_of(mu, r);
+        Mat<3, float> t = product<DF>(U, g, x, mu, r, nu, df);
+        if (r < ND - 1) t = mul_nd(t, load_link<3, float, DF>(U, g, x, nu, df));
+        part[r] = t;
+      }
+    } else {
+      p += mu * NT;
+      if (gl < ND - 1) fwd[gl] = mul_nd(p[gl], load_link<3, float, DF>(U, g, x, nu_of(mu, gl), df));
+    }
+    __syncwarp(mask);
+    Mat<3, float> S = mzero<3, float>();
+#pragma unroll 1
+    for (int k = 0; k < ND - 1; ++k) madd(S, DF ? p[k] : fwd[k]);
+#pragma unroll 1
+    for (int k = ND - 1; k < NT; ++k) madd(S, p[k]);
+    return S;
+  }
+};
+
+// The links of site x in the order mu = 0 .. Nd-1; hits(S, U, dlink) updates one link
+// and returns its accepted hits, the same in every lane.
+template <int ND, bool DF, int G, typename Hits>
+KLFT_D int group_links(StapleTerms<ND> &sh, const Links<3, float> &U, const Geom &g, const Site &x, const Defect &df,
+                       Hits &&hits) {
+  const long long lx = site_lin(g, x);
+  const int gl = (int)(threadIdx.x & (unsigned)(G - 1));
+  const unsigned mask = group_mask<G>();
+  sh.template load<DF, G>(U, g, x, df, gl);
+  __syncwarp(mask);
+  const bool own0 = DF && df.active && in_defect(g, df, x, 0);
+  int nacc = 0;
+#pragma unroll 1
+  for (int mu = 0; mu < ND; ++mu) {
+    if (open_link(g, x, mu)) continue;
+    const Mat<3, float> S = sh.template staple<DF, G>(U, g, x, mu, df, gl, mask);
+    Mat<3, float> V = U.load(lx, mu);
+    const int n = hits(S, V, mu == 0 && own0);
+    __syncwarp(mask);  // every lane has read the link and the terms
+    if (n && gl == 0) U.store(lx, mu, V);
+    __syncwarp(mask);
+    nacc += n;
+  }
+  return nacc;
+}
+
+// The same from shared parts.
+template <int ND, bool DF, int G, int NC, typename T, typename Hits>
 KLFT_D int group_links(StapleParts<NC, ND, T> &sh, const Links<NC, T> &U, const Geom &g, const Site &x,
                        const Defect &df, Hits &&hits) {
   const long long lx = site_lin(g, x);
@@ -295,7 +377,7 @@ KLFT_D int group_links(StapleParts<NC, ND, T> &sh, const Links<NC, T> &U, const 
       __syncwarp(mask);
       if (gl == 0) {
         U.store(lx, mu, V);
-        sh.own[mu] = as_stored<NC, T>(V);
+        sh.own[mu] = V;
       }
       __syncwarp(mask);
     }
@@ -396,7 +478,8 @@ template <int NC, int ND, typename T, int G> struct GroupShared {
   DrawTable<NC, T, G> table;
   StapleParts<NC, SharedStaples<NC, T>::v ? ND : 1, T> parts;
 };
-template <int ND, typename T, int G> struct GroupShared<3, ND, T, G> { StapleParts<3, ND, T> parts; };
+template <int ND, int G> struct GroupShared<3, ND, double, G> { StapleParts<3, ND, double> parts; };
+template <int ND, int G> struct GroupShared<3, ND, float, G> { StapleTerms<ND> parts; };
 
 // Site t (if t < Vh) of class val by the calling thread's group; sh: one entry per
 // group of the CTA.  Every thread of the CTA calls it and passes the wait.  The
@@ -418,7 +501,7 @@ KLFT_D int group_site_update(GroupShared<NC, ND, T, G> *shared, const Links<NC, 
     grid_dependency_wait();
     grid_launch_dependents();
     if (ok)
-      n = group_links<3, ND, T, DF, G>(sh.parts, U, g, x, df, [&](const Mat<3, T> &S, Mat<3, T> &V, bool dlink) {
+      n = group_links<ND, DF, G>(sh.parts, U, g, x, df, [&](const Mat<3, T> &S, Mat<3, T> &V, bool dlink) {
         return lanes.hits(S, V, bnc, dlink, dlink ? (T)defect_c(df) : T(1));
       });
   } else {
@@ -428,7 +511,7 @@ KLFT_D int group_site_update(GroupShared<NC, ND, T, G> *shared, const Links<NC, 
     grid_launch_dependents();
     if (ok) {
       if constexpr (SharedStaples<NC, T>::v) {
-        n = group_links<NC, ND, T, DF, G>(sh.parts, U, g, x, df, [&](const Mat<NC, T> &S, Mat<NC, T> &V, bool dlink) {
+        n = group_links<ND, DF, G>(sh.parts, U, g, x, df, [&](const Mat<NC, T> &S, Mat<NC, T> &V, bool dlink) {
           return group_hits<NC>(S, V, a, dlink, df, rng, bnc);
         });
       } else {

@@ -102,3 +102,26 @@ def test_fp32_group_pass_resumes_hits_and_orders_stores(nc, L, nhits):
     np.testing.assert_array_equal(alone.metropolis(BETA[nc], DELTA[nc], nhits, 4), acc[:, 0])
     np.testing.assert_array_equal(alone.download(), member.download())
     b.close()
+
+
+# SU(3) in FP32 where many hits are accepted (strong coupling, disordered links) and 10^8 are
+# drawn: a staple whose last bit differs changes one decision in 10^7
+@pytest.mark.parametrize("L,defect,beta", [([16, 16, 12, 12], 0, 0.5), ([16, 16, 12, 12], 0, 2.0),
+                                           ([16, 16, 12, 12], 2, 2.0), ([24, 20, 36], 0, 1.0)])
+def test_su3_fp32_group_pass_at_strong_coupling(L, defect, beta):
+    big = [24, 24, 24, 32] if len(L) == 4 else [64, 56, 56]
+    fields = []
+    for ext, seed in ((L, 5), (L, 5), (big, 6)):
+        g = GaugeField(ext, 3, "mixed", "hot", seed)
+        g.set_stream(seed, 1)
+        if defect:
+            g.set_defect(defect, (0, 1, 0), 0.5)
+        fields.append(g)
+    alone, member, other = fields
+    b = Batch()
+    for g in (member, other):
+        b.add(g, beta, 0.1, 40)
+    acc, _, _, _ = b.run(20, False, False)
+    np.testing.assert_array_equal(alone.metropolis(beta, 0.1, 40, 20), acc[:, 0])
+    np.testing.assert_array_equal(alone.download(), member.download())
+    b.close()
