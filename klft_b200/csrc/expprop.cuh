@@ -50,8 +50,8 @@ template <typename V> struct XMat { V re[3][3], im[3][3]; };
 // (d c0, a + d c1, b), and exp(iQ) = f0 + f1 Q + f2 Q^2 with
 // f = sum_n i^n / n! (a_n, b_n, d_n).  Arguments with c1 > 3/4 (an eigenvalue
 // possibly above 1: |lambda|^2 <= 4 c1 / 3) are scaled by 2^-k and the result
-// squared k times in coefficient space, all in the basis of the scaled Q (c0, c1
-// its own):
+// squared k times in coefficient space, the basis and c0, c1 taken from Q to 2 Q
+// after each:
 //   (f0 + f1 Q + f2 Q^2)^2 = (f0^2 + 2 f1 f2 c0) + (2 f0 f1 + 2 f1 f2 c1 + f2^2 c0) Q
 //                          + (f1^2 + 2 f0 f2 + f2^2 c1) Q^2.
 template <typename V> KLFT_D XMat<V> expi_gellmann(const V h[8], V s) {
@@ -77,16 +77,15 @@ template <typename V> KLFT_D XMat<V> expi_gellmann(const V h[8], V s) {
   c0 = vfma(splat<V>(2.0), re3, c0);
   c0 = vsub(c0, vfma(d0, n12, vfma(d1, n02, vmul(d2, n01))));
   int sq = 0;
-  V cs1 = c1, cs0 = c0, scale = splat<V>(1.0);
+  V cs1 = c1, cs0 = c0;
   float big = (float)vmax(c1);
   while (big > 0.75f && sq < 64) {  // halve Q: c1 / 4, c0 / 8
     cs1 = vmul(cs1, splat<V>(0.25));
     cs0 = vmul(cs0, splat<V>(0.125));
-    scale = vmul(scale, splat<V>(0.5));
     big *= 0.25f;
     ++sq;
   }
-  // Taylor sum of exp(i Q'), Q' = scale Q, in the basis (1, Q', Q'^2)
+  // Taylor sum of exp(i Q'), Q' = 2^-sq Q, in the basis (1, Q', Q'^2)
   V ta = splat<V>(1.0), tb = splat<V>(0.0), td = splat<V>(0.0);
   V f0r = splat<V>(1.0), f0i = splat<V>(0.0), f1r = splat<V>(0.0), f1i = splat<V>(0.0), f2r = splat<V>(0.0),
     f2i = splat<V>(0.0);
@@ -122,15 +121,12 @@ template <typename V> KLFT_D XMat<V> expi_gellmann(const V h[8], V s) {
                                        vsub(vmul(f1r, f1r), vmul(f1i, f1i))));
     const V g2i = vfma(f22i, cs1, vfma(splat<V>(2.0), vfma(f0r, f2i, vmul(f0i, f2r)),
                                        vmul(splat<V>(2.0), vmul(f1r, f1i))));
-    f0r = g0r; f0i = g0i; f1r = g1r; f1i = g1i; f2r = g2r; f2i = g2i;
-  }
-  // back to the basis (1, Q, Q^2): Q' = scale Q
-  if (sq) {
-    const V sc2 = vmul(scale, scale);
-    f1r = vmul(f1r, scale);
-    f1i = vmul(f1i, scale);
-    f2r = vmul(f2r, sc2);
-    f2i = vmul(f2i, sc2);
+    // from the basis (1, Q', Q'^2) to that of 2 Q'
+    f0r = g0r; f0i = g0i;
+    f1r = vmul(splat<V>(0.5), g1r); f1i = vmul(splat<V>(0.5), g1i);
+    f2r = vmul(splat<V>(0.25), g2r); f2i = vmul(splat<V>(0.25), g2i);
+    cs1 = vmul(cs1, splat<V>(4.0));
+    cs0 = vmul(cs0, splat<V>(8.0));
   }
   // Q^2 (hermitian): diagonal and upper triangle
   const V s00 = vfma(d0, d0, vadd(n01, n02));
